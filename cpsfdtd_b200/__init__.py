@@ -646,7 +646,7 @@ def footprint(dk, precision=FP32) -> int:
     total = 6 * cells * esz + cells
     if dk.pml:
         n = dk.pml["npml"]
-        xw = sum((v + 32) // 32 * 32 for v in n[0:2] if v) * (ny + 1) * (nz + 1)
+        xw = sum((v + 39) // 32 * 32 for v in n[0:2] if v) * (ny + 1) * (nz + 1)
         yw = sum(v + 1 for v in n[2:4] if v) * px * (nz + 1)
         zw = sum(v + 1 for v in n[4:6] if v) * px * (ny + 1)
         total += 2 * 2 * esz * (xw + yw + zw)  # two psi per slab cell for E and for H

@@ -34,7 +34,7 @@ struct GridSig {
     int64_t step;
     const void *f0, *dl, *gain, *st, *q, *tg0, *tg1, *srcw, *ring0;
     int64_t dl_n, g_n;
-    int nports, nsrc, ntg0, ntg1, pml, by;
+    int nports, nsrc, ntg0, ntg1, pml, by, kc;
     int64_t nfreq_sum;
     bool operator==(const GridSig &o) const { return memcmp(this, &o, sizeof(GridSig)) == 0; }
 };
@@ -50,7 +50,7 @@ GridSig signature(const cps_grid *g)
     s.dl_n = g->dl_on ? g->dl_n : -1; s.g_n = g->gain_on ? g->g_n : -1;
     s.nports = (int)g->ports.size(); s.nsrc = (int)g->src.size();
     s.ntg0 = g->tfsf_on ? g->ntg[0] : -1; s.ntg1 = g->tfsf_on ? g->ntg[1] : -1;
-    s.pml = g->pml_on; s.by = g->tma_by;
+    s.pml = g->pml_on; s.by = g->tma_by; s.kc = g->shape.kc;
     for (const PortState &P : g->ports) s.nfreq_sum += P.nfreq * 7 + P.npts;
     return s;
 }
@@ -87,8 +87,8 @@ struct cps_batch {
     bool dirty = true;
     // configuration
     int by = 4, kc = 16, persistent = 2, graph = 1;  // per-member launches: fastest on the measured mixes
-    int kch = 0;  // planes per tile of the per-member H sweeps (0: kc)
-    int kcg = 0;  // planes per tile of the per-member FP32 E sweeps with gain (0: kc)
+    bool tile_set = false;   // tiling set by the caller: it holds for the per-member launches too
+    bool grid_tiles = false; // a grid's internal one-grid batch: its own tile shape
     // device tables (owned)
     std::vector<void *> owned;
     void *d_grids = nullptr;
@@ -254,7 +254,7 @@ cps_status rebuild_T(cps_batch *b)
         CK(cudaStreamSynchronize(g->stream));
         BatchGrid<T> &B = hg[gi];
         memset((void *)&B, 0, sizeof(B));
-        B.M = g->tma;
+        B.M = g->tma.t;
         B.f = field_view<T>(g);
         B.p = pml_view<T>(g);
         B.D = dl_view<T>(g);
@@ -389,6 +389,23 @@ cps_status rebuild_T(cps_batch *b)
     return CPS_OK;
 }
 
+// Tile shape of a member's own sweep launches: the batch's when the caller set
+// it, the grid's own in a one-grid batch; else the grid's planes as they are
+// (members run beside one another, so a small one need not fill the device)
+// and the batch's for the E sweep with gain.
+FusedShape member_shape(const cps_batch *b, const cps_grid *g)
+{
+    FusedShape sh = g->shape;
+    if (b->tile_set) {
+        sh = FusedShape{b->by, b->kc};
+        sh.fixed = true;
+    } else if (!b->grid_tiles) {
+        sh.kcg = b->kc;
+        sh.fixed = true;
+    }
+    return sh;
+}
+
 // Enqueue one chunk of S steps on the batch stream; returns the launch count.
 template <typename T>
 int64_t enqueue_chunk(cps_batch *b, int S)
@@ -402,8 +419,7 @@ int64_t enqueue_chunk(cps_batch *b, int S)
         launch_h_batch<T>(G, b->d_tiles[kHPml], b->ntiles[kHPml], b->nblocks[kHPml], b->by, true, b->d_err, st);
         per_member(b, [&](int gi, cudaStream_t ms) {
             const cps_grid *g = b->grids[gi];
-            n += launch_h_tma<T>(g->tma, field_view<T>(g), pml_view<T>(g), FusedShape{b->by, b->kc, b->kch}, b->d_err,
-                                 ms);
+            n += launch_h_tma<T>(g->tma, field_view<T>(g), pml_view<T>(g), member_shape(b, g), b->d_err, ms);
         });
         launch_inject_batch<T>(G, b->d_inj[1], b->ninj[1], 1, s, st);
         for (int c = 0; c < 8; ++c)
@@ -412,7 +428,7 @@ int64_t enqueue_chunk(cps_batch *b, int S)
         per_member(b, [&](int gi, cudaStream_t ms) {
             const cps_grid *g = b->grids[gi];
             n += launch_e_tma<T>(g->tma, field_view<T>(g), pml_view<T>(g), dl_view<T>(g), gain_view<T>(g),
-                            FusedShape{b->by, b->kc, 0, b->kcg}, b->d_err, ms, &g->lane);
+                            member_shape(b, g), b->d_err, ms, &g->lane);
         });
         launch_inject_batch<T>(G, b->d_inj[0], b->ninj[0], 0, s, st);
         launch_sources_batch<T>(G, b->d_src, b->nsrc, s, st);
@@ -547,13 +563,11 @@ bool cache_lookup(const char *path, const std::string &key, int *by, int *kc, in
 
 }  // namespace
 
-void cps::batch_set_h_planes(cps_batch *b, int kch, int kcg)
+void cps::batch_use_grid_tiles(cps_batch *b)
 {
-    if (b->kch != kch || b->kcg != kcg) {
-        b->kch = kch;
-        b->kcg = kcg;
-        b->dirty = true;  // captured chunks launch the per-member sweeps with them
-    }
+    if (b->tile_set) b->dirty = true;  // captured chunks launch the per-member sweeps with the tiling
+    b->tile_set = false;
+    b->grid_tiles = true;
 }
 
 // clears a batch's device error word (the grid reset of a grid stepped
@@ -649,9 +663,9 @@ extern "C" cps_status cps_batch_set_tile(cps_batch *b, int32_t rows, int32_t pla
     REQUIRE(rows == 4 || rows == 8, CPS_E_INVALID, "cps_batch_set_tile: rows must be 4 or 8");
     REQUIRE(planes >= 1 && planes <= 4096, CPS_E_INVALID, "cps_batch_set_tile: planes out of range");
     REQUIRE(persistent >= 0 && persistent <= 2, CPS_E_INVALID, "cps_batch_set_tile: persistent is 0, 1 or 2");
-    if (b->by != rows || b->kc != planes || b->persistent != persistent) {
+    if (b->by != rows || b->kc != planes || b->persistent != persistent || !b->tile_set) {
         b->by = rows; b->kc = planes; b->persistent = persistent;
-        b->dirty = true;
+        b->tile_set = b->dirty = true;
     }
     return CPS_OK;
 }

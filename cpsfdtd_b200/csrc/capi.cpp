@@ -77,6 +77,14 @@ cps_status dalloc(cps_grid *g, void **p, size_t bytes)
     return CPS_OK;
 }
 
+// n arrays of `bytes` each (a multiple of 128), one after another in one allocation
+cps_status dalloc_run(cps_grid *g, void **p, int n, size_t bytes)
+{
+    cps_status s = dalloc(g, p, (size_t)n * bytes);
+    for (int q = 1; q < n && !s; ++q) p[q] = (char *)p[0] + (size_t)q * bytes;
+    return s;
+}
+
 void dfree(cps_grid *g, void *p)
 {
     if (!p) return;
@@ -397,22 +405,23 @@ cps_status ensure_tma(cps_grid *g)
     EncodeTiled enc = encode_fn();
     REQUIRE(enc, CPS_E_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
     const Dims &d = g->d;
+    TmaMaps &T = g->tma.t;
     const cuuint64_t dims[3] = {(cuuint64_t)d.px, (cuuint64_t)(d.ny + 1), (cuuint64_t)(d.nz + 1)};
     const cuuint32_t es[3] = {1, 1, 1};
     const CUtensorMapDataType dt = g->fp32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64;
     const cuuint64_t st[2] = {(cuuint64_t)d.px * g->esz, (cuuint64_t)d.pxy * g->esz};
     const cuuint32_t halo[3] = {36, (cuuint32_t)by + 1, 1}, own[3] = {32, (cuuint32_t)by, 1};
     for (int c = 0; c < 6; ++c) {
-        CUresult r1 = enc(&g->tma.halo[c], dt, 3, g->F[c], dims, st, halo, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+        CUresult r1 = enc(&T.halo[c], dt, 3, g->F[c], dims, st, halo, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
                           CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        CUresult r2 = enc(&g->tma.own[c], dt, 3, g->F[c], dims, st, own, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+        CUresult r2 = enc(&T.own[c], dt, 3, g->F[c], dims, st, own, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
                           CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         REQUIRE(r1 == CUDA_SUCCESS && r2 == CUDA_SUCCESS, CPS_E_CUDA, "cuTensorMapEncodeTiled failed for a field");
     }
     const cuuint64_t sid[2] = {(cuuint64_t)d.px, (cuuint64_t)d.pxy};
-    CUresult r = enc(&g->tma.id, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, g->d_id, dims, sid, own, es,
+    CUresult r = enc(&T.id, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, g->d_id, dims, sid, own, es,
                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     REQUIRE(r == CUDA_SUCCESS, CPS_E_CUDA, "cuTensorMapEncodeTiled failed for the IDs");
@@ -424,10 +433,42 @@ cps_status ensure_tma(cps_grid *g)
         const cuuint64_t gst[4] = {32 * sizeof(float), seg_b, nseg * seg_b, nseg * seg_b * (cuuint64_t)(d.ny + 1)};
         const cuuint32_t gbox[5] = {32, (cuuint32_t)kGainPersist, 1, (cuuint32_t)by, 1};
         const cuuint32_t ges[5] = {1, 1, 1, 1, 1};
-        r = enc(&g->tma.gain, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 5, g->d_g_state, gdims, gst, gbox, ges,
+        r = enc(&T.gain, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 5, g->d_g_state, gdims, gst, gbox, ges,
                 CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         REQUIRE(r == CUDA_SUCCESS, CPS_E_CUDA, "cuTensorMapEncodeTiled failed for the gain words");
+    }
+    // one-grid sweeps: boxes over the three components of a side (contiguous arrays)
+    auto encode = [&](CUtensorMap *m, CUtensorMapDataType type, int rank, void *base, const cuuint64_t *dim,
+                      const cuuint64_t *stride, const cuuint32_t *box) {
+        const cuuint32_t one[5] = {1, 1, 1, 1, 1};
+        return enc(m, type, rank, base, dim, stride, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                   CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    };
+    const cuuint64_t fd[4] = {dims[0], dims[1], dims[2], 3}, fs[3] = {st[0], st[1], (cuuint64_t)g->elems * g->esz};
+    for (int side = 0; side < 2; ++side) {  // 0: H sweep, 1: E sweep
+        SweepMaps &W = side == 0 ? g->tma.h : g->tma.e;
+        void *other = g->F[side == 0 ? 0 : 3], *swept = g->F[side == 0 ? 3 : 0];
+        for (cuuint32_t P = 1; P <= 2; ++P) {
+            const cuuint32_t hb[4] = {36, (cuuint32_t)by + 1, P, 3}, ob[4] = {32, (cuuint32_t)by, P, 3};
+            REQUIRE(encode(&W.halo[P - 1], dt, 4, other, fd, fs, hb) == CUDA_SUCCESS &&
+                        encode(&W.own[P - 1], dt, 4, swept, fd, fs, ob) == CUDA_SUCCESS &&
+                        encode(&W.id[P - 1], CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, g->d_id, dims, sid, ob) == CUDA_SUCCESS,
+                    CPS_E_CUDA, "cuTensorMapEncodeTiled failed for a side's fields");
+        }
+        const cuuint32_t tb[4] = {36, (cuuint32_t)by + 1, 1, 2};
+        REQUIRE(encode(&W.tail, dt, 4, other, fd, fs, tb) == CUDA_SUCCESS, CPS_E_CUDA,
+                "cuTensorMapEncodeTiled failed for a side's fields");
+        W.gain = T.gain;
+        for (int f = 0; f < 6 && g->pml_on; ++f) {
+            const cuuint64_t np = (cuuint64_t)g->pml.npml[f];
+            const cuuint64_t row = f < 2 ? (cuuint64_t)psi_xw((int)np) : (cuuint64_t)d.px;
+            const cuuint64_t pd[4] = {row, f / 2 == 1 ? np + 1 : dims[1], f < 4 ? dims[2] : np + 1, 2};
+            const cuuint64_t ps[3] = {row * g->esz, row * pd[1] * g->esz, (cuuint64_t)psi_words(g, f) * g->esz};
+            const cuuint32_t pb[4] = {32, (cuuint32_t)by, 1, 2};
+            REQUIRE(encode(&W.psi[f], dt, 4, g->d_q[f][side == 0 ? 2 : 0], pd, ps, pb) == CUDA_SUCCESS, CPS_E_CUDA,
+                    "cuTensorMapEncodeTiled failed for the CPML psi words");
+        }
     }
     g->tma_by = by;
     return CPS_OK;
@@ -466,18 +507,17 @@ cps_status ensure_onepass(cps_grid *g)
     cps_status s;
     if (!g->F2[0]) {
         // zeroed once: the sweep writes every cell of the arrays, never the x padding
-        for (int c = 0; c < 6; ++c) {
-            if ((s = dalloc(g, &g->F2[c], (size_t)g->elems * g->esz))) return s;
-            CK(cudaMemsetAsync(g->F2[c], 0, (size_t)g->elems * g->esz, g->stream));
+        for (int c = 0; c < 6; c += 3) {
+            if ((s = dalloc_run(g, &g->F2[c], 3, (size_t)g->elems * g->esz))) return s;
+            CK(cudaMemsetAsync(g->F2[c], 0, 3 * (size_t)g->elems * g->esz, g->stream));
         }
     }
     if (g->pml_on && !g->d_q2[0][0]) {
-        for (int f = 0; f < 6; ++f)
-            for (int q = 0; q < 2; ++q) {
-                const size_t n = psi_words(g, f) * g->esz;
-                if ((s = dalloc(g, &g->d_q2[f][q], n))) return s;
-                CK(cudaMemsetAsync(g->d_q2[f][q], 0, n, g->stream));
-            }
+        for (int f = 0; f < 6; ++f) {
+            const size_t n = psi_words(g, f) * g->esz;
+            if ((s = dalloc_run(g, &g->d_q2[f][0], 2, n))) return s;
+            CK(cudaMemsetAsync(g->d_q2[f][0], 0, 2 * n, g->stream));
+        }
     }
     if (g->tfsf_on && g->ntg[1] > 0 && !g->d_hslot && g->hc_ok) {
         // each H-side contribution's slot in the per-face arrays of the targets' bounding box
@@ -734,6 +774,7 @@ extern "C" cps_status cps_grid_create(const cps_grid_desc *desc, cps_grid **out)
     if (!(g->desc.dt > 0)) g->desc.dt = cps_courant_dt(desc->dx, desc->dy, desc->dz);
     g->fp32 = desc->precision == CPS_FP32;
     g->esz = g->fp32 ? 4 : 8;
+    if (!g->fp32) g->shape.kch = 16;
     g->d.nx = desc->nx; g->d.ny = desc->ny; g->d.nz = desc->nz;
     g->d.px = (desc->nx + 1 + kXPad - 1) / kXPad * kXPad;
     g->d.pxy = (int64_t)g->d.px * (desc->ny + 1);
@@ -746,7 +787,8 @@ extern "C" cps_status cps_grid_create(const cps_grid_desc *desc, cps_grid **out)
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&g->lane.join, cudaEventDisableTiming);
     if (e != cudaSuccess) { set_error(cudaGetErrorString(e)); cps_grid_destroy(g); return CPS_E_CUDA; }
     cps_status s = CPS_OK;
-    for (int c = 0; c < 6 && !s; ++c) s = dalloc(g, &g->F[c], (size_t)g->elems * g->esz);
+    // the three components of a side lie one after another (one tensor map covers them)
+    for (int c = 0; c < 6 && !s; c += 3) s = dalloc_run(g, &g->F[c], 3, (size_t)g->elems * g->esz);
     if (!s) s = dalloc(g, (void **)&g->d_id, (size_t)g->elems);
     if (!s) s = dalloc(g, &g->d_media, 4 * 256 * g->esz);
     if (!s) s = dalloc(g, (void **)&g->d_counter, sizeof(unsigned long long));
@@ -991,16 +1033,13 @@ extern "C" cps_status cps_pml_init(cps_grid *g, const cps_pml_params *pp)
     if ((s = upload_real(g, g->d_pcoef, coef.data(), coef.size()))) return s;
     const Dims &d = g->d;
     for (int f = 0; f < 6; ++f) {
-        const int np = pp->npml[f];
-        size_t n;
-        if (f < 2) n = (size_t)(d.nz + 1) * (d.ny + 1) * psi_xw(np);
-        else if (f < 4) n = (size_t)(d.nz + 1) * (np + 1) * d.px;
-        else n = (size_t)(np + 1) * (d.ny + 1) * d.px;
-        for (int q = 0; q < 4; ++q)
-            if ((s = dalloc(g, &g->d_q[f][q], n * g->esz))) return s;
+        // each side's two words lie one after the other (one tensor map covers them)
+        for (int q = 0; q < 4; q += 2)
+            if ((s = dalloc_run(g, &g->d_q[f][q], 2, psi_words(g, f) * g->esz))) return s;
     }
     if ((s = push_stretch(g))) return s;
     g->pml_on = true;
+    g->tma_by = 0;  // the sweeps' tensor maps now include the psi words
     return CPS_OK;
 }
 
@@ -1573,7 +1612,7 @@ cps_status solo_step(cps_grid *g, int32_t nsteps)
     if ((rows != g->shape.by || planes != g->shape.kc || pers != 0) &&
         (s = cps_batch_set_tile(g->solo, g->shape.by, g->shape.kc, 0)))
         return s;
-    batch_set_h_planes(g->solo, g->shape.kch, g->shape.kcg);
+    batch_use_grid_tiles(g->solo);
     int64_t l0 = 0, l1 = 0;
     cps_batch_launch_count(g->solo, &l0);
     s = cps_batch_step(g->solo, nsteps);
@@ -2165,6 +2204,7 @@ extern "C" cps_status cps_grid_set_tile(cps_grid *g, int32_t rows, int32_t plane
     g->shape.kc = planes;
     g->shape.kch = planes;
     g->shape.kcg = planes;
+    g->shape.fixed = true;
     return CPS_OK;
 }
 

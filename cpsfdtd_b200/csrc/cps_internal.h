@@ -36,9 +36,13 @@ constexpr double kEps0 = 8.8541878176E-12;
 constexpr double kQe = -1.602176565E-19;  // electron charge
 constexpr double kMe = 9.10938215E-31;    // electron mass
 
-// row width of an x-slab psi array ([k][j][s], s = 0..np): np+1 rounded up to
-// 32 words so every row starts on a 128-byte line
-__host__ __device__ inline int psi_xw(int np) { return (np + 32) / 32 * 32; }
+// row width of an x-slab psi array ([k][j][s], s = 0..np): whole 128-byte lines
+// with room for the second end's shift (psi_shift) and for the last vector of
+// cells to run past the slab
+__host__ __device__ inline int psi_xw(int np) { return (np + 8 + 31) / 32 * 32; }
+// words in front of s = 0 in a row of the second x end, so that word s of cell
+// i = nx - np + s lies on a 16-byte boundary whenever i is a multiple of 4
+__host__ __device__ inline int psi_shift(int nx, int np) { return (nx - np) & 3; }
 
 struct Dims {
     int nx, ny, nz;   // cells
@@ -270,6 +274,7 @@ struct FusedShape {
     int kc;       // planes per block along z (E sweep; H sweep too when kch is 0)
     int kch = 0;  // planes per block of the TMA H sweep (0: kc)
     int kcg = 0;  // planes per block of an FP32 TMA E sweep with gain (0: kc)
+    bool fixed = false;  // asked for by the caller (else fewer planes on small grids)
 };
 // A second stream of a grid with a fork and a join event: work that does not
 // depend on a sweep (the Drude-Lorentz cell pass beside the E sweep) runs on
@@ -292,13 +297,13 @@ namespace cps {
 // (each sweep launches its CPML tiles and its interior tiles separately;
 // the return value is the number of kernels launched)
 template <typename T>
-int launch_h_tma(const TmaMaps &M, const FieldView<T> &f, const PmlView<T> &p, FusedShape sh, int *err,
+int launch_h_tma(const GridMaps &M, const FieldView<T> &f, const PmlView<T> &p, FusedShape sh, int *err,
                  cudaStream_t s);
 // With a side lane, the Drude-Lorentz cell pass runs on it beside the E sweep
 // (the sweep leaves the ID-2 cells, their E and their psi alone, and both
 // read only H and the cells' own old E); the call returns after the join.
 template <typename T>
-int launch_e_tma(const TmaMaps &M, const FieldView<T> &f, const PmlView<T> &p, const DlView<T> &D,
+int launch_e_tma(const GridMaps &M, const FieldView<T> &f, const PmlView<T> &p, const DlView<T> &D,
                  const GainView<T> &G, FusedShape sh, int *err, cudaStream_t s, const SideLane *lane = nullptr);
 // set the shared-memory attributes of every TMA sweep kernel (call outside captures)
 template <typename T>

@@ -74,7 +74,6 @@ struct cps_grid {
     using InjTarget = cps::InjTarget;
     using InjContrib = cps::InjContrib;
     using FusedShape = cps::FusedShape;
-    using TmaMaps = cps::TmaMaps;
     using StepMaps = cps::StepMaps;
     template <typename T> using DlCoef = cps::DlCoef<T>;
     cps_grid_desc desc{};
@@ -150,14 +149,14 @@ struct cps_grid {
     // misc
     int64_t step = 1;
     int64_t launches = 0;
-    // the E sweep's tiles march 8 planes, the H sweep's 16 and an FP32 E
-    // sweep with gain 4 (measured fastest on the laser and dispersive decks);
-    // cps_grid_set_tile sets all three
-    FusedShape shape{4, 8, 16, 4};
+    // tiles march 8 planes, in the FP64 H sweep 16 (cps_grid_create) and in an
+    // FP32 E sweep with gain 4 (measured fastest on the laser and dispersive
+    // decks), fewer on small grids; cps_grid_set_tile sets all three
+    FusedShape shape{4, 8, 8, 4};
     double *d_conv = nullptr;
     unsigned long long *d_counter = nullptr;
     // TMA tensor maps of the fused sweeps (built for tile rows tma_by)
-    TmaMaps tma{};
+    cps::GridMaps tma{};
     int tma_by = 0;
     int sweep_mode = 0;  // 0: TMA-fed sweeps, 1: register sweeps
     // one-pass step (CPS_PATH_ONEPASS): a second field buffer and H-side psi
@@ -270,8 +269,9 @@ inline PmlView<T> pml_view(const cps_grid *g)
         p.cE[f] = c + off; off += n;
         p.bH[f] = c + off; off += n;
         p.cH[f] = c + off; off += n;
-        p.qe[f][0] = (T *)g->d_q[f][0]; p.qe[f][1] = (T *)g->d_q[f][1];
-        p.qh[f][0] = (T *)g->d_q[f][2]; p.qh[f][1] = (T *)g->d_q[f][3];
+        const int o = f == kFX2 ? psi_shift(g->d.nx, p.np[f]) : 0;
+        p.qe[f][0] = (T *)g->d_q[f][0] + o; p.qe[f][1] = (T *)g->d_q[f][1] + o;
+        p.qh[f][0] = (T *)g->d_q[f][2] + o; p.qh[f][1] = (T *)g->d_q[f][3] + o;
     }
     p.cpmlE = (T)g->cpmlE;
     p.cpmlH = (T)g->cpmlH;
@@ -287,8 +287,9 @@ inline PmlView<T> pml_view_alt(const cps_grid *g)
     PmlView<T> p = pml_view<T>(g);
     if (p.on)
         for (int f = 0; f < 6; ++f) {
-            p.qh[f][0] = (T *)g->d_q2[f][0];
-            p.qh[f][1] = (T *)g->d_q2[f][1];
+            const int o = f == kFX2 ? psi_shift(g->d.nx, p.np[f]) : 0;
+            p.qh[f][0] = (T *)g->d_q2[f][0] + o;
+            p.qh[f][1] = (T *)g->d_q2[f][1] + o;
         }
     return p;
 }
@@ -346,8 +347,7 @@ inline ThreeView three_view(const cps_grid *g)
 
 // clears the device error word of a batch (batch.cpp)
 cps_status batch_clear_error(cps_batch *b);
-// planes per tile of the H sweeps and of the FP32 E sweeps with gain that a
-// batch launches per member (0: its kc)
-void batch_set_h_planes(cps_batch *b, int kch, int kcg = 0);
+// per-member launches of a batch take each grid's own tile shape
+void batch_use_grid_tiles(cps_batch *b);
 
 }  // namespace cps

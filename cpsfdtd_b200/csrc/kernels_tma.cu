@@ -5,7 +5,7 @@
 
 #include <algorithm>
 
-#include "tma_bodies.cuh"
+#include "warp_tiles.cuh"
 
 namespace cps {
 
@@ -41,6 +41,7 @@ __global__ void __launch_bounds__(32 * BY, GAIN ? 512 / (32 * BY) : 1024 / (32 *
         e_tma_body<T, BY, false, DL, GAIN>(M, f, p, D, G, kc, t, ctr, err, sm, full);
 }
 
+// FP64 H sweep (block tiles): one launch, the body each tile needs (PM 2)
 template <typename T, int BY, int PM>
 __global__ void __launch_bounds__(32 * BY) k_h_tma(const __grid_constant__ TmaMaps M, FieldView<T> f, PmlView<T> p,
                                                     int kc, const __grid_constant__ TileBoxes tb, int *err)
@@ -57,6 +58,53 @@ __global__ void __launch_bounds__(32 * BY) k_h_tma(const __grid_constant__ TmaMa
         h_tma_body<T, BY, PM != 0>(M, f, p, kc, t, ctr, err, sm, full);
     else
         h_tma_body<T, BY, false>(M, f, p, kc, t, ctr, err, sm, full);
+}
+
+// blocks of one warp that fit an SM's shared memory
+template <typename T, int BY, bool GAIN>
+constexpr int warp_blocks()
+{
+    return (227 * 1024) / (warp_ring<T, BY, GAIN>() + 1024 + 640);
+}
+
+// One warp per tile.  PM: 0 no CPML on the grid, 2 the body each tile needs.
+template <typename T, int BY, int PM>
+__global__ void __launch_bounds__(32, warp_blocks<T, BY, false>())
+    k_h_warp(const __grid_constant__ SweepMaps M, FieldView<T> f, PmlView<T> p, int kc, int nbx, int nby, int *err)
+{
+    extern __shared__ __align__(128) unsigned char sm_raw[];
+    __shared__ __align__(8) uint64_t full[kMaxStages];
+    const TileXYZ t = grid_tile((int)blockIdx.x, nbx, nby);
+    const int k0 = t.bz * kc, k1 = min(k0 + kc, f.d.nz);
+    if (k0 >= k1) return;
+    __shared__ Coef2<T> tab[kTab];
+    if (threadIdx.x < kTab) tab[threadIdx.x] = Coef2<T>{f.aH[threadIdx.x], f.bH[threadIdx.x]};
+    init_ring(full);
+    Ring R{align_smem(sm_raw), full, warp_ring<T, BY, false>() - 128, 0u, wait_skew(err), err};
+    if (PM == 1 || (PM == 2 && tile_in_pml(p.np, f.d, t.bx * 32, t.by * BY, BY, k0, k1, false)))
+        h_warp_tile<T, BY, 1, PM != 0>(M, f, p, kc, t, R, tab);
+    else
+        h_warp_tile<T, BY, kPlanes, false>(M, f, p, kc, t, R, tab);
+}
+
+template <typename T, int BY, int PM, bool DL, bool GAIN>
+__global__ void __launch_bounds__(32, warp_blocks<T, BY, GAIN>())
+    k_e_warp(const __grid_constant__ SweepMaps M, FieldView<T> f, PmlView<T> p, GainView<T> G, int kc, int nbx, int nby,
+             int *err)
+{
+    extern __shared__ __align__(128) unsigned char sm_raw[];
+    __shared__ __align__(8) uint64_t full[kMaxStages];
+    const TileXYZ t = grid_tile((int)blockIdx.x, nbx, nby);
+    const int k0 = max(1, t.bz * kc), k1 = min(t.bz * kc + kc, f.d.nz);
+    if (k0 >= k1) return;
+    __shared__ Coef2<T> tab[kTab];
+    if (threadIdx.x < kTab) tab[threadIdx.x] = Coef2<T>{f.aE[threadIdx.x], f.bE[threadIdx.x]};
+    init_ring(full);
+    Ring R{align_smem(sm_raw), full, warp_ring<T, BY, GAIN>() - 128, 0u, wait_skew(err), err};
+    if (PM == 1 || (PM == 2 && tile_in_pml(p.np, f.d, t.bx * 32, t.by * BY, BY, k0, k1, true)))
+        e_warp_tile<T, BY, 1, PM != 0, DL, GAIN>(M, f, p, G, kc, t, R, tab);
+    else
+        e_warp_tile<T, BY, GAIN ? 1 : kPlanes, false, DL, GAIN>(M, f, p, G, kc, t, R, tab);
 }
 
 // The ID-2 cells the TMA E sweep leaves alone, one thread per cell of the
@@ -172,68 +220,111 @@ int h_tma_launch(const TmaMaps &M, const FieldView<T> &f, const PmlView<T> &p, i
     return 1;
 }
 
-// the kernels the launchers below use (CPML-free, per-tile, and for gain the
-// two halves of the split)
+template <typename T, int BY, int PM>
+int h_warp_launch(const SweepMaps &M, const FieldView<T> &f, const PmlView<T> &p, int kc, int *err, cudaStream_t s)
+{
+    kc = (kc + kPlanes - 1) / kPlanes * kPlanes;
+    constexpr int smem = warp_ring<T, BY, false>();
+    const int nbx = (int)cdiv(f.d.nx, 32), nby = (int)cdiv(f.d.ny, BY), nbz = (int)cdiv(f.d.nz, kc);
+    if (!set_smem<k_h_warp<T, BY, PM>>(smem)) return 0;
+    k_h_warp<T, BY, PM><<<nbx * nby * nbz, 32, smem, s>>>(M, f, p, kc, nbx, nby, err);
+    return 1;
+}
+
+template <typename T, int BY, int PM, bool DL, bool GAIN>
+int e_warp_launch(const SweepMaps &M, const FieldView<T> &f, const PmlView<T> &p, const GainView<T> &G, int kc, int *err,
+                  cudaStream_t s)
+{
+    kc = (kc + kPlanes - 1) / kPlanes * kPlanes;
+    constexpr int smem = warp_ring<T, BY, GAIN>();
+    const int nbx = (int)cdiv(f.d.nx, 32), nby = (int)cdiv(f.d.ny, BY), nbz = (int)cdiv(f.d.nz, kc);
+    if (!set_smem<k_e_warp<T, BY, PM, DL, GAIN>>(smem)) return 0;
+    k_e_warp<T, BY, PM, DL, GAIN><<<nbx * nby * nbz, 32, smem, s>>>(M, f, p, G, kc, nbx, nby, err);
+    return 1;
+}
+
+// the kernels the launchers below use
 template <typename T, int BY>
 void attrs_by()
 {
-    constexpr int S = StageLayout<T, BY>::SMEM, SG = StageLayout<T, BY, sizeof(T) == 4>::SMEM;
-    set_smem<k_h_tma<T, BY, 0>>(S);
-    set_smem<k_h_tma<T, BY, 2>>(S);
-    set_smem<k_e_tma<T, BY, 0, false, false>>(S);
+    constexpr int S = warp_ring<T, BY, false>(), SB = StageLayout<T, BY>::SMEM;
+    constexpr int SG = StageLayout<T, BY, sizeof(T) == 4>::SMEM;
+    if constexpr (sizeof(T) == 4) {
+        set_smem<k_h_warp<T, BY, 0>>(S);
+        set_smem<k_h_warp<T, BY, 2>>(S);
+    } else {
+        set_smem<k_h_tma<T, BY, 0>>(SB);
+        set_smem<k_h_tma<T, BY, 2>>(SB);
+    }
+    set_smem<k_e_warp<T, BY, 0, false, false>>(S);
+    set_smem<k_e_warp<T, BY, 0, true, false>>(S);
+    set_smem<k_e_warp<T, BY, 2, false, false>>(S);
+    set_smem<k_e_warp<T, BY, 2, true, false>>(S);
     set_smem<k_e_tma<T, BY, 0, false, true>>(SG);
-    set_smem<k_e_tma<T, BY, 0, true, false>>(S);
     set_smem<k_e_tma<T, BY, 0, true, true>>(SG);
-    set_smem<k_e_tma<T, BY, 2, false, false>>(S);
-    set_smem<k_e_tma<T, BY, 2, true, false>>(S);
     set_smem<k_e_tma<T, BY, 1, false, true>>(SG);
     set_smem<k_e_tma<T, BY, 1, true, true>>(SG);
 }
 
 template <typename T, int BY>
-int e_tma_by(const TmaMaps &M, const FieldView<T> &f, const PmlView<T> &p, const DlView<T> &D,
+int e_tma_by(const GridMaps &M, const FieldView<T> &f, const PmlView<T> &p, const DlView<T> &D,
              const GainView<T> &G, int kc, int *err, cudaStream_t s)
 {
     const bool dl = D.on && D.ncell > 0, gn = G.on && G.ncell > 0;
-    const SweepTiles t = sweep_tiles(p.np, p.on, f.d, BY, kc, true);
     if (gn && sizeof(T) == 4 && p.on) {  // every tile on the CPML body, one launch
         const TileBoxes all = whole_grid(f.d, BY, kc);
-        return dl ? e_tma_launch<T, BY, 1, true, true>(M, f, p, D, G, kc, all, err, s)
-                  : e_tma_launch<T, BY, 1, false, true>(M, f, p, D, G, kc, all, err, s);
+        return dl ? e_tma_launch<T, BY, 1, true, true>(M.t, f, p, D, G, kc, all, err, s)
+                  : e_tma_launch<T, BY, 1, false, true>(M.t, f, p, D, G, kc, all, err, s);
     }
     if (gn) {  // CPML tiles (if any) and interior tiles as two launches
-        return (dl ? e_tma_launch<T, BY, 1, true, true>(M, f, p, D, G, kc, t.pml, err, s)
-                   : e_tma_launch<T, BY, 1, false, true>(M, f, p, D, G, kc, t.pml, err, s)) +
-               (dl ? e_tma_launch<T, BY, 0, true, true>(M, f, p, D, G, kc, t.interior, err, s)
-                   : e_tma_launch<T, BY, 0, false, true>(M, f, p, D, G, kc, t.interior, err, s));
+        const SweepTiles t = sweep_tiles(p.np, p.on, f.d, BY, kc, true);
+        return (dl ? e_tma_launch<T, BY, 1, true, true>(M.t, f, p, D, G, kc, t.pml, err, s)
+                   : e_tma_launch<T, BY, 1, false, true>(M.t, f, p, D, G, kc, t.pml, err, s)) +
+               (dl ? e_tma_launch<T, BY, 0, true, true>(M.t, f, p, D, G, kc, t.interior, err, s)
+                   : e_tma_launch<T, BY, 0, false, true>(M.t, f, p, D, G, kc, t.interior, err, s));
     }
-    const TileBoxes all = whole_grid(f.d, BY, kc);
     if (p.on)
-        return dl ? e_tma_launch<T, BY, 2, true, false>(M, f, p, D, G, kc, all, err, s)
-                  : e_tma_launch<T, BY, 2, false, false>(M, f, p, D, G, kc, all, err, s);
-    return dl ? e_tma_launch<T, BY, 0, true, false>(M, f, p, D, G, kc, all, err, s)
-              : e_tma_launch<T, BY, 0, false, false>(M, f, p, D, G, kc, all, err, s);
+        return dl ? e_warp_launch<T, BY, 2, true, false>(M.e, f, p, G, kc, err, s)
+                  : e_warp_launch<T, BY, 2, false, false>(M.e, f, p, G, kc, err, s);
+    return dl ? e_warp_launch<T, BY, 0, true, false>(M.e, f, p, G, kc, err, s)
+              : e_warp_launch<T, BY, 0, false, false>(M.e, f, p, G, kc, err, s);
 }
 
 template <typename T, int BY>
-int h_tma_by(const TmaMaps &M, const FieldView<T> &f, const PmlView<T> &p, int kc, int *err, cudaStream_t s)
+int h_tma_by(const GridMaps &M, const FieldView<T> &f, const PmlView<T> &p, int kc, int *err, cudaStream_t s)
 {
-    const TileBoxes all = whole_grid(f.d, BY, kc);
-    return p.on ? h_tma_launch<T, BY, 2>(M, f, p, kc, all, err, s) : h_tma_launch<T, BY, 0>(M, f, p, kc, all, err, s);
+    if constexpr (sizeof(T) == 8) {
+        const TileBoxes all = whole_grid(f.d, BY, kc);
+        return p.on ? h_tma_launch<T, BY, 2>(M.t, f, p, kc, all, err, s) : h_tma_launch<T, BY, 0>(M.t, f, p, kc, all, err, s);
+    } else {
+        return p.on ? h_warp_launch<T, BY, 2>(M.h, f, p, kc, err, s) : h_warp_launch<T, BY, 0>(M.h, f, p, kc, err, s);
+    }
 }
 
 }  // namespace
 
+// Planes per tile: as set, or the sweep's default, halved (to two at least)
+// while the grid has fewer tiles than the device holds at once (14 one-warp
+// tiles per SM, five block tiles).  A tile marches its planes one after the
+// other, so on a small grid the sweep takes the time of one tile: at 48^3, H
+// and E sweeps of 22 and 14 us with 16 and 8 planes.
+static int planes(int kc, const FusedShape &sh, const Dims &d, bool warp)
+{
+    const int64_t cols = (int64_t)cdiv(d.nx, 32) * cdiv(d.ny, sh.by), want = 148 * (warp ? 14 : 5);
+    while (!sh.fixed && kc > 2 && cols * cdiv(d.nz, kc) < want) kc /= 2;
+    return kc;
+}
+
 template <typename T>
-int launch_h_tma(const TmaMaps &M, const FieldView<T> &f, const PmlView<T> &p, FusedShape sh, int *err,
+int launch_h_tma(const GridMaps &M, const FieldView<T> &f, const PmlView<T> &p, FusedShape sh, int *err,
                  cudaStream_t s)
 {
-    const int kc = sh.kch > 0 ? sh.kch : sh.kc;
+    const int kc = planes(sh.kch > 0 ? sh.kch : sh.kc, sh, f.d, sizeof(T) == 4);
     return sh.by == 4 ? h_tma_by<T, 4>(M, f, p, kc, err, s) : h_tma_by<T, 8>(M, f, p, kc, err, s);
 }
 
 template <typename T>
-int launch_e_tma(const TmaMaps &M, const FieldView<T> &f, const PmlView<T> &p, const DlView<T> &D,
+int launch_e_tma(const GridMaps &M, const FieldView<T> &f, const PmlView<T> &p, const DlView<T> &D,
                  const GainView<T> &G, FusedShape sh, int *err, cudaStream_t s, const SideLane *lane)
 {
     const bool dl = D.on && D.ncell > 0;
@@ -248,11 +339,9 @@ int launch_e_tma(const TmaMaps &M, const FieldView<T> &f, const PmlView<T> &p, c
         if (p.on) k_dl_cells<T, true><<<cdiv(D.ncell, 128), 128, 0, ds>>>(f, p, D);
         else k_dl_cells<T, false><<<cdiv(D.ncell, 128), 128, 0, ds>>>(f, p, D);
     }
-    // an FP32 sweep with gain takes its own plane count (4 by default: with
-    // its three-stage ring of large stages it ran 1.9 % faster on 4-plane
-    // tiles than on 8 on the 384^3 laser deck, while the E sweep without gain
-    // ran 9 % slower on 4 than on 8 on the 256^3 dispersive deck)
-    const int kc = G.on && G.ncell > 0 && sizeof(T) == 4 && sh.kcg > 0 ? sh.kcg : sh.kc;
+    // an FP32 sweep with gain takes its own plane count
+    const bool gn = G.on && G.ncell > 0;
+    const int kc = planes(gn && sizeof(T) == 4 && sh.kcg > 0 ? sh.kcg : sh.kc, sh, f.d, !gn);
     const int n = sh.by == 4 ? e_tma_by<T, 4>(M, f, p, D, G, kc, err, s) : e_tma_by<T, 8>(M, f, p, D, G, kc, err, s);
     if (beside) {
         cudaEventRecord(lane->join, lane->s);
@@ -270,14 +359,14 @@ void tma_attributes()
 
 template void tma_attributes<float>();
 template void tma_attributes<double>();
-template int launch_h_tma<float>(const TmaMaps &, const FieldView<float> &, const PmlView<float> &, FusedShape, int *,
+template int launch_h_tma<float>(const GridMaps &, const FieldView<float> &, const PmlView<float> &, FusedShape, int *,
                                   cudaStream_t);
-template int launch_h_tma<double>(const TmaMaps &, const FieldView<double> &, const PmlView<double> &, FusedShape,
+template int launch_h_tma<double>(const GridMaps &, const FieldView<double> &, const PmlView<double> &, FusedShape,
                                    int *, cudaStream_t);
-template int launch_e_tma<float>(const TmaMaps &, const FieldView<float> &, const PmlView<float> &,
+template int launch_e_tma<float>(const GridMaps &, const FieldView<float> &, const PmlView<float> &,
                                   const DlView<float> &, const GainView<float> &, FusedShape, int *, cudaStream_t,
                                   const SideLane *);
-template int launch_e_tma<double>(const TmaMaps &, const FieldView<double> &, const PmlView<double> &,
+template int launch_e_tma<double>(const GridMaps &, const FieldView<double> &, const PmlView<double> &,
                                    const DlView<double> &, const GainView<double> &, FusedShape, int *, cudaStream_t,
                                    const SideLane *);
 

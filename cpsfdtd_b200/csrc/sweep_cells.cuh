@@ -8,6 +8,42 @@
 
 namespace cps {
 
+// Rounding written out: one product, one sum or one fused multiply-add each, so
+// that every kernel that holds an update computes the same bits, whatever the
+// compiler would contract around it.
+__device__ __forceinline__ float rmul(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double rmul(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float radd(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ double radd(double a, double b) { return __dadd_rn(a, b); }
+__device__ __forceinline__ float rfma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double rfma(double a, double b, double c) { return __fma_rn(a, b, c); }
+
+// a F + b d1 c1 - b d2 c2 (bulk E and H updates, BasicFDTD.cpp:25-84)
+template <typename T>
+__device__ __forceinline__ T yee(T a, T F, T b, T d1, T c1, T d2, T c2)
+{
+    return rfma(-rmul(b, d2), c2, rfma(a, F, rmul(rmul(b, d1), c1)));
+}
+// the same in the Hz update's order of rounding
+template <typename T>
+__device__ __forceinline__ T yee_z(T a, T F, T b, T d1, T c1, T d2, T c2)
+{
+    return rfma(-rmul(b, d2), c2, rfma(rmul(b, d1), c1, rmul(a, F)));
+}
+// a F - b d1 c1 + b d2 c2
+template <typename T>
+__device__ __forceinline__ T yee_n(T a, T F, T b, T d1, T c1, T d2, T c2)
+{
+    return rfma(rmul(b, d2), c2, rfma(a, F, -rmul(rmul(b, d1), c1)));
+}
+// b psi + c d, and a component with +/- psi times its curl coefficient
+template <typename T>
+__device__ __forceinline__ T psi_new(T b, T psi, T c, T d) { return rfma(b, psi, rmul(c, d)); }
+template <typename T>
+__device__ __forceinline__ T psi_add(T F, T a, T cc) { return rfma(a, cc, F); }
+template <typename T>
+__device__ __forceinline__ T psi_sub(T F, T a, T cc) { return rfma(-a, cc, F); }
+
 __device__ __forceinline__ unsigned lanemask_lt()
 {
     unsigned m;
@@ -98,19 +134,19 @@ __device__ __forceinline__ void pml_e_cell(const PmlView<T> &p, const Dims &d, c
         const int np = p.np[c.fx];
         const int64_t q = ((int64_t)k * (d.ny + 1) + j) * psi_xw(np) + c.sxl;
         T *q0 = p.qe[c.fx][0], *q1 = p.qe[c.fx][1];
-        const T a0 = c.bx * q0[q] + c.cx * dHz_i, a1 = c.bx * q1[q] + c.cx * dHy_i;
+        const T a0 = psi_new(c.bx, q0[q], c.cx, dHz_i), a1 = psi_new(c.bx, q1[q], c.cx, dHy_i);
         q0[q] = a0; q1[q] = a1;
-        ey = ey - a0 * ce;
-        ez = ez + a1 * ce;
+        ey = psi_sub(ey, a0, ce);
+        ez = psi_add(ez, a1, ce);
     }
     if (c.fy >= 0) {
         const int np = p.np[c.fy];
         const int64_t q = ((int64_t)k * (np + 1) + c.syl) * d.px + i;
         T *q0 = p.qe[c.fy][0], *q1 = p.qe[c.fy][1];
-        const T a0 = c.by * q0[q] + c.cy * dHx_j, a1 = c.by * q1[q] + c.cy * dHz_j;
+        const T a0 = psi_new(c.by, q0[q], c.cy, dHx_j), a1 = psi_new(c.by, q1[q], c.cy, dHz_j);
         q0[q] = a0; q1[q] = a1;
-        ez = ez - a0 * ce;
-        ex = ex + a1 * ce;
+        ez = psi_sub(ez, a0, ce);
+        ex = psi_add(ex, a1, ce);
     }
     int fz = -1, szl = 0;
     if (k <= p.np[kFZ1]) { fz = kFZ1; szl = k; }
@@ -119,10 +155,10 @@ __device__ __forceinline__ void pml_e_cell(const PmlView<T> &p, const Dims &d, c
         const int64_t q = ((int64_t)szl * (d.ny + 1) + j) * d.px + i;
         T *q0 = p.qe[fz][0], *q1 = p.qe[fz][1];
         const T b = p.bE[fz][szl], cc = p.cE[fz][szl];
-        const T a0 = b * q0[q] + cc * dHy_k, a1 = b * q1[q] + cc * dHx_k;
+        const T a0 = psi_new(b, q0[q], cc, dHy_k), a1 = psi_new(b, q1[q], cc, dHx_k);
         q0[q] = a0; q1[q] = a1;
-        ex = ex - a0 * ce;
-        ey = ey + a1 * ce;
+        ex = psi_sub(ex, a0, ce);
+        ey = psi_add(ey, a1, ce);
     }
 }
 
@@ -184,17 +220,17 @@ __device__ __forceinline__ void pml_e_cell_pre(const PmlView<T> &p, const Dims &
 {
     if (c.fx >= 0) {
         const int64_t q = ((int64_t)k * (d.ny + 1) + j) * psi_xw(p.np[c.fx]) + c.sxl;
-        const T a0 = c.bx * r.x0 + c.cx * dHz_i, a1 = c.bx * r.x1 + c.cx * dHy_i;
+        const T a0 = psi_new(c.bx, r.x0, c.cx, dHz_i), a1 = psi_new(c.bx, r.x1, c.cx, dHy_i);
         p.qe[c.fx][0][q] = a0; p.qe[c.fx][1][q] = a1;
-        ey = ey - a0 * ce;
-        ez = ez + a1 * ce;
+        ey = psi_sub(ey, a0, ce);
+        ez = psi_add(ez, a1, ce);
     }
     if (c.fy >= 0) {
         const int64_t q = ((int64_t)k * (p.np[c.fy] + 1) + c.syl) * d.px + i;
-        const T a0 = c.by * r.y0 + c.cy * dHx_j, a1 = c.by * r.y1 + c.cy * dHz_j;
+        const T a0 = psi_new(c.by, r.y0, c.cy, dHx_j), a1 = psi_new(c.by, r.y1, c.cy, dHz_j);
         p.qe[c.fy][0][q] = a0; p.qe[c.fy][1][q] = a1;
-        ez = ez - a0 * ce;
-        ex = ex + a1 * ce;
+        ez = psi_sub(ez, a0, ce);
+        ex = psi_add(ex, a1, ce);
     }
     int fz = -1, szl = 0;
     if (k <= p.np[kFZ1]) { fz = kFZ1; szl = k; }
@@ -202,10 +238,10 @@ __device__ __forceinline__ void pml_e_cell_pre(const PmlView<T> &p, const Dims &
     if (fz >= 0) {
         const int64_t q = ((int64_t)szl * (d.ny + 1) + j) * d.px + i;
         const T b = p.bE[fz][szl], cc = p.cE[fz][szl];
-        const T a0 = b * r.z0 + cc * dHy_k, a1 = b * r.z1 + cc * dHx_k;
+        const T a0 = psi_new(b, r.z0, cc, dHy_k), a1 = psi_new(b, r.z1, cc, dHx_k);
         p.qe[fz][0][q] = a0; p.qe[fz][1][q] = a1;
-        ex = ex - a0 * ce;
-        ey = ey + a1 * ce;
+        ex = psi_sub(ex, a0, ce);
+        ey = psi_add(ey, a1, ce);
     }
 }
 
@@ -218,17 +254,17 @@ __device__ __forceinline__ void pml_h_cell_pre(const PmlView<T> &p, const Dims &
 {
     if (c.fx >= 0) {
         const int64_t q = ((int64_t)k * (d.ny + 1) + j) * psi_xw(p.np[c.fx]) + c.sxl;
-        const T a0 = c.bx * r.x0 + c.cx * dEz_i, a1 = c.bx * r.x1 + c.cx * dEy_i;
+        const T a0 = psi_new(c.bx, r.x0, c.cx, dEz_i), a1 = psi_new(c.bx, r.x1, c.cx, dEy_i);
         if (STORE && store) { p.qh[c.fx][0][q] = a0; p.qh[c.fx][1][q] = a1; }
-        hy = hy + a0 * ch;
-        hz = hz - a1 * ch;
+        hy = psi_add(hy, a0, ch);
+        hz = psi_sub(hz, a1, ch);
     }
     if (c.fy >= 0) {
         const int64_t q = ((int64_t)k * (p.np[c.fy] + 1) + c.syl) * d.px + i;
-        const T a0 = c.by * r.y0 + c.cy * dEx_j, a1 = c.by * r.y1 + c.cy * dEz_j;
+        const T a0 = psi_new(c.by, r.y0, c.cy, dEx_j), a1 = psi_new(c.by, r.y1, c.cy, dEz_j);
         if (STORE && store) { p.qh[c.fy][0][q] = a0; p.qh[c.fy][1][q] = a1; }
-        hz = hz - a0 * ch;
-        hx = hx + a1 * ch;
+        hz = psi_sub(hz, a0, ch);
+        hx = psi_add(hx, a1, ch);
     }
     int fz = -1, szl = 0;
     if (k < p.np[kFZ1]) { fz = kFZ1; szl = k; }
@@ -236,11 +272,37 @@ __device__ __forceinline__ void pml_h_cell_pre(const PmlView<T> &p, const Dims &
     if (fz >= 0) {
         const int64_t q = ((int64_t)szl * (d.ny + 1) + j) * d.px + i;
         const T b = p.bH[fz][szl], cc = p.cH[fz][szl];
-        const T a0 = b * r.z0 + cc * dEy_k, a1 = b * r.z1 + cc * dEx_k;
+        const T a0 = psi_new(b, r.z0, cc, dEy_k), a1 = psi_new(b, r.z1, cc, dEx_k);
         if (STORE && store) { p.qh[fz][0][q] = a0; p.qh[fz][1][q] = a1; }
-        hx = hx - a0 * ch;
-        hy = hy + a1 * ch;
+        hx = psi_sub(hx, a0, ch);
+        hy = psi_add(hy, a1, ch);
     }
+}
+
+// dl_component for compile-time pole counts, from state words already in
+// registers (w[0 .. ND+2NL], the component's words in order)
+template <typename T, int ND, int NL>
+__device__ __forceinline__ T dl_component_regs(const DlCoef<T> &D, T E, T curl, const T *w, T *st, int64_t sc)
+{
+    const T temp = E;
+    T t1 = T(0), t2 = T(0);
+#pragma unroll
+    for (int p = 0; p < ND; ++p) t1 = rfma(D.C4[p], w[p], t1);
+#pragma unroll
+    for (int p = 0; p < NL; ++p) t2 = rfma(D.C6[p], w[ND + NL + p], rfma(D.C5[p], w[ND + p], t2));
+    const T e1 = w[ND + 2 * NL];
+    E = radd(radd(radd(rfma(D.C1, E, rmul(D.C2, e1)), curl), -t1), -t2);
+#pragma unroll
+    for (int p = 0; p < ND; ++p) st[p * sc] = rfma(D.kappa[p], w[p], rmul(D.beta[p], E + temp));
+#pragma unroll
+    for (int p = 0; p < NL; ++p) {
+        const T t0 = w[ND + p];
+        st[(ND + p) * sc] =
+            radd(rfma(D.alpha[p], t0, rmul(D.xi[p], w[ND + NL + p])), rmul(D.gammaL[p], E - e1) / T(2.0) / D.dt);
+        st[(ND + NL + p) * sc] = t0;
+    }
+    st[(ND + 2 * NL) * sc] = temp;
+    return E;
 }
 
 // Drude-Lorentz update of the ID-2 cells of a warp row (ballot-ranked lookup
@@ -369,34 +431,63 @@ __device__ __forceinline__ void gain_staged32(const float *ws, GainRegs32 &r)
     r.n[2] = ws[L::N3 * 32];
 }
 
+// one component of the gain update at a cell: P (FourLevelLaser.cpp:274-295,
+// words scaled by CEP), E -= dP (:302-305); E1 is the field before
+__device__ __forceinline__ void gain_comp32(const GainCoef &G, float E1, float dNa, float dNb, float pa, float pa1,
+                                            float pb, float pb1, float &a, float &b, float &E)
+{
+    a = rfma(rmul(E1, G.fa3), dNa, rfma(G.fa1, pa, rmul(G.fa2, pa1)));
+    b = rfma(rmul(E1, G.fb3), dNb, rfma(G.fb1, pb, rmul(G.fb2, pb1)));
+    E = E1 - radd(radd(radd(a, -pa), b), -pb);
+}
+
+// population offsets from the energy-exchange sums (gain_n_update<float>)
+__device__ __forceinline__ void gain_pops32(const GainCoef &G, float sa, float sb, float s2, float m0, float &n1,
+                                            float &n2, float &n3)
+{
+    const float q3 = rfma(G.k3a, 1.0f - n2, -rmul(G.k3b, m0));
+    const float n3n = rfma(G.fpump, 1.0f + m0, __fdividef(rfma(n3, 1.0f - q3, rmul(G.hb, sb)), 1.0f + q3));
+    const float q1 = rfma(G.k1a, n2, -rmul(G.k1b, m0));
+    const float n1n = __fdividef(rfma(-G.ha, sa, rfma(n1, 1.0f - q1, rmul(2.0f * G.k1b, m0))), 1.0f + q1);
+    const float q2 = rfma(G.k3a, n3n, -rmul(G.k1a, n1n));
+    const float n2n = __fdividef(rfma(G.ha, s2, rfma(n2, 1.0f - q2, rmul(2.0f * G.k3a, n3n))), 1.0f + q2);
+    n1 = n1n;
+    n2 = n2n;
+    n3 = n3n;
+}
+
 // P -> E -> N at a gain cell (device index g) from its words r; the new words
-// go to the dense state
+// go to the dense state.  The Ey term of the N2 sum uses P - P' as the
+// reference does (FourLevelLaser.cpp:316).
 __device__ __forceinline__ void gain_apply32(const GainView<float> &G, int64_t g, const GainRegs32 &r, float &ex,
                                              float &ey, float &ez)
 {
     using L = GainSite32;
     float *st = G.state + gain_dense_index(g);
     const int64_t sc = kGainGroup;
-    float E[3] = {ex, ey, ez}, E1[3] = {ex, ey, ez};
-    float Pa[3], Pa1[3], Pa2[3], Pb[3], Pb1[3], Pb2[3];
+    float n1 = r.n[0], n2 = r.n[1], n3 = r.n[2];
+    const float m0 = conserve_m0(n1, n2, n3);  // FP64 conservation, FourLevelLaser.cpp:324
+    const float dNa = (n2 - n1) - 1.0f, dNb = (n3 - m0) - 1.0f;
+    float sa = 0.0f, sb = 0.0f, s2 = 0.0f;
 #pragma unroll
-    for (int q = 0; q < 3; ++q) { Pa[q] = r.pa[q]; Pa1[q] = r.pa1[q]; Pb[q] = r.pb[q]; Pb1[q] = r.pb1[q]; }
-    Pops<float> N;
-    N.n1 = r.n[0];
-    N.n2 = r.n[1];
-    N.n3 = r.n[2];
-    N.m0 = conserve_m0(N.n1, N.n2, N.n3);  // FP64 conservation, FourLevelLaser.cpp:324
-    gain_p_update<float>(G.c, N, E, Pa, Pa1, Pa2, Pb, Pb1, Pb2);
-#pragma unroll
-    for (int q = 0; q < 3; ++q) E[q] = gain_e_corr<float>(G.c, E[q], Pa[q], Pa1[q], Pb[q], Pb1[q]);
-    gain_n_update<float>(G.c, N, E, E1, Pa, Pa1, Pa2, Pb, Pb2);
-#pragma unroll
-    for (int q = 0; q < 3; ++q) {
-        st[(L::PA + q) * sc] = Pa[q]; st[(L::PA1 + q) * sc] = Pa1[q];
-        st[(L::PB + q) * sc] = Pb[q]; st[(L::PB1 + q) * sc] = Pb1[q];
+    for (int o = 0; o < 3; ++o) {
+        const int q = o == 0 ? 1 : o == 1 ? 0 : 2;
+        float &F = q == 0 ? ex : q == 1 ? ey : ez;
+        const float E1 = F;
+        float a, b, E;
+        gain_comp32(G.c, E1, dNa, dNb, r.pa[q], r.pa1[q], r.pb[q], r.pb1[q], a, b, E);
+        const float da = a - r.pa1[q], db = b - r.pb1[q], d2 = q == 1 ? a - r.pa[q] : da;
+        sa = o == 0 ? rmul(E1, da) : rfma(E1, da, sa);
+        sb = o == 0 ? rmul(E1, db) : rfma(E1, db, sb);
+        s2 = o == 0 ? rmul(E + E1, d2) : rfma(E + E1, d2, s2);
+        st[(L::PA + q) * sc] = a; st[(L::PA1 + q) * sc] = r.pa[q];
+        st[(L::PB + q) * sc] = b; st[(L::PB1 + q) * sc] = r.pb[q];
+        F = E;
     }
-    gain_store_n<float>(st, sc, N);
-    ex = E[0]; ey = E[1]; ez = E[2];
+    gain_pops32(G.c, sa, sb, s2, m0, n1, n2, n3);
+    st[L::DN1 * sc] = n1;
+    st[L::N2 * sc] = n2;
+    st[L::N3 * sc] = n3;
 }
 
 }  // namespace cps

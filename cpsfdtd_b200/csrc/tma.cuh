@@ -19,6 +19,29 @@ struct TmaMaps {
     CUtensorMap gain;
 };
 
+// Tensor maps one one-grid sweep reads, index P - 1 for stages of P planes:
+//   halo  the other side's components {px, ny+1, nz+1, 3}, box 36 x (BY+1) x P x 3
+//   own   the swept side's, box 32 x BY x P x 3
+//   id    the IDs {px, ny+1, nz+1}, box 32 x BY x P
+//   tail  Ex and Ey of one plane, box 36 x (BY+1) x 1 x 2 (H sweep)
+//   gain  the gain words (as TmaMaps::gain)
+//   psi   by face, the side's two words, box 32 x BY x 1 x 2: x slabs {row
+//         words, ny+1, nz+1, 2}, y slabs {px, np+1, nz+1, 2}, z slabs {px, ny+1, np+1, 2}
+struct SweepMaps {
+    CUtensorMap halo[2];
+    CUtensorMap own[2];
+    CUtensorMap id[2];
+    CUtensorMap tail;
+    CUtensorMap gain;
+    CUtensorMap psi[6];
+};
+
+// every map of a grid's sweeps
+struct GridMaps {
+    TmaMaps t;       // block-tile kernels (the batch's tables)
+    SweepMaps h, e;  // one-grid H and E sweeps
+};
+
 // Tensor maps of the one-pass step sweep over one field buffer, x fastest:
 //   e[c]: Ex Ey Ez, box 40 x (BY+2) x 1 (from x0-4, y0-1)
 //   h[c]: Hx Hy Hz, box 36 x (BY+1) x 1 (from x0-4, y0-1)
@@ -76,6 +99,17 @@ __device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, u
         "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
         " [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(smem_u32(dst)),
         "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z)
+        : "memory");
+}
+
+// 4-D tiled load (components outermost), completion counted on bar
+__device__ __forceinline__ void tma_load_4d(void *dst, const CUtensorMap *map, uint64_t *bar, int c0, int c1, int c2,
+                                            int c3)
+{
+    asm volatile(
+        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+        " [%0], [%1, {%3, %4, %5, %6}], [%2];" ::"r"(smem_u32(dst)),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
         : "memory");
 }
 

@@ -233,9 +233,9 @@ __device__ __forceinline__ bool e_tma_body(const TmaMaps &M, const FieldView<T> 
             ex = T(0); ey = T(0); ez = T(0);
         } else if (id != CPS_ID_DISPERSIVE) {
             const T aE = __ldg(&f.aE[id]), bE = __ldg(&f.bE[id]);
-            ex = aE * ex + bE * dHz_j * cExz - bE * dHy_k * cExy;
-            ey = aE * ey + bE * dHx_k * cEyx - bE * dHz_i * cEyz;
-            ez = aE * ez + bE * dHy_i * cEzy - bE * dHx_j * cEzx;
+            ex = yee(aE, ex, bE, dHz_j, cExz, dHy_k, cExy);
+            ey = yee(aE, ey, bE, dHx_k, cEyx, dHz_i, cEyz);
+            ez = yee(aE, ez, bE, dHy_i, cEzy, dHx_j, cEzx);
         }
         if constexpr (GST) {
             // the gain list holds interior cells only (act), with the gain ID
@@ -344,9 +344,9 @@ __device__ __forceinline__ bool h_tma_body(const TmaMaps &M, const FieldView<T> 
             const T dEx_k = exk - ex, dEy_k = eyk - ey;
             const int id = idt[orow];
             const T aH = __ldg(&f.aH[id]), bH = __ldg(&f.bH[id]);
-            T hx = aH * hxt[orow] - bH * dEz_j * cHxz + bH * dEy_k * sv.cHxy[k];
-            T hy = aH * hyt[orow] - bH * dEx_k * sv.cHyx[k] + bH * dEz_i * cHyz;
-            T hz = aH * hzt[orow] + bH * dEx_j * cHzx - bH * dEy_i * cHzy;
+            T hx = yee_n(aH, hxt[orow], bH, dEz_j, cHxz, dEy_k, sv.cHxy[k]);
+            T hy = yee_n(aH, hyt[orow], bH, dEx_k, sv.cHyx[k], dEz_i, cHyz);
+            T hz = yee_z(aH, hzt[orow], bH, dEx_j, cHzx, dEy_i, cHzy);
             if (act) {
                 if (PML)
                     pml_h_cell_pre(p, d, pc, pml_ch_cell(p, f.bH, id), i, j, k, qc, dEz_i, dEy_i, dEx_j, dEz_j, dEy_k,
@@ -395,9 +395,9 @@ __device__ __forceinline__ void dl_cell(const FieldView<T> &f, const FieldView<T
     const StretchView<T> &s = f.s;
     const T cExz = s.cExz[j], cEzx = s.cEzx[j], cEyz = s.cEyz[i], cEzy = s.cEzy[i], cExy = s.cExy[k], cEyx = s.cEyx[k];
     const T C3 = D.c.C3;
-    const T cxx = C3 * dHz_j * cExz - C3 * dHy_k * cExy;
-    const T cyy = C3 * dHx_k * cEyx - C3 * dHz_i * cEyz;
-    const T czz = C3 * dHy_i * cEzy - C3 * dHx_j * cEzx;
+    const T cxx = rfma(rmul(C3, dHz_j), cExz, -rmul(rmul(C3, dHy_k), cExy));
+    const T cyy = rfma(rmul(C3, dHx_k), cEyx, -rmul(rmul(C3, dHz_i), cEyz));
+    const T czz = rfma(rmul(C3, dHy_i), cEzy, -rmul(rmul(C3, dHx_j), cEzx));
     const int64_t sc = D.ncell;
     T *st = D.state + c;
     T ex = fo.Ex[g], ey = fo.Ey[g], ez = fo.Ez[g];
