@@ -621,6 +621,28 @@ cps_status check_device_error(cps_grid *g)
     return CPS_OK;
 }
 
+// whether a TF/SF target or a source may lie in a CPML slab (E slabs reach
+// index np, one further than H slabs; H targets lie one cell outside the box)
+bool tfsf_meets_pml(const cps_grid *g)
+{
+    for (int f = 0; f < 6; ++f)
+        if (g->tp.n[f] - 1 <= g->pml.npml[f]) return true;
+    return false;
+}
+
+bool sources_meet_pml(const cps_grid *g)
+{
+    const Dims &d = g->d;
+    const int n[3] = {d.nx, d.ny, d.nz};
+    for (const Src &s : g->src) {
+        const int k = (int)(s.idx / d.pxy), j = (int)((s.idx - k * d.pxy) / d.px);
+        const int at[3] = {(int)(s.idx - k * d.pxy - (int64_t)j * d.px), j, k};
+        for (int a = 0; a < 3; ++a)
+            if (at[a] <= g->pml.npml[2 * a] || at[a] >= n[a] - g->pml.npml[2 * a + 1]) return true;
+    }
+    return false;
+}
+
 template <typename T>
 cps_status step_T(cps_grid *g, int nsteps, int path)
 {
@@ -637,13 +659,17 @@ cps_status step_T(cps_grid *g, int nsteps, int path)
     const PmlView<T> p = pml_view<T>(g);
     const DlView<T> D = dl_view<T>(g);
     const GainView<T> G = gain_view<T>(g);
+    // plain path: a side's bulk update and CPML routine in one launch where no
+    // routine between them touches a slab cell
+    const bool h_with_pml = g->pml_on && !(g->tfsf_on && tfsf_meets_pml(g));
+    const bool e_with_pml = h_with_pml && !g->dl_on && !g->gain_on && !g->three_on && !sources_meet_pml(g);
     for (int it = 0; it < nsteps; ++it) {
         const int64_t n = g->step;
         if (path == CPS_PATH_PLAIN) {
-            launch_h_bulk<T>(f, g->stream);
+            launch_h_bulk<T>(f, p, h_with_pml, g->stream);
             op_inject<T>(g, 1, (double)n, CPS_FACE_ALL);
-            if (g->pml_on) launch_h_pml<T>(f, p, g->stream);
-            launch_e_bulk<T>(f, g->stream);
+            if (g->pml_on && !h_with_pml) launch_h_pml<T>(f, p, g->stream);
+            launch_e_bulk<T>(f, p, e_with_pml, g->stream);
             if (g->dl_on) launch_dl<T>(f, D, g->stream);
             if (g->gain_on) {
                 launch_gain<T>(f, G, 0, g->stream);
@@ -659,8 +685,8 @@ cps_status step_T(cps_grid *g, int nsteps, int path)
             }
             op_inject<T>(g, 0, (double)n, CPS_FACE_ALL);
             op_sources<T>(g, (int)n);
-            if (g->pml_on) launch_e_pml<T>(f, p, g->stream);
-            g->launches += 2 + (g->pml_on ? 12 : 0) + (g->dl_on ? 1 : 0) + (g->gain_on ? 3 : 0);
+            if (g->pml_on && !e_with_pml) launch_e_pml<T>(f, p, g->stream);
+            g->launches += 2 + (g->pml_on ? 2 - h_with_pml - e_with_pml : 0) + (g->dl_on ? 1 : 0) + (g->gain_on ? 3 : 0);
         } else if (onepass) {
             // one sweep into the other buffers, which become current; then the
             // Drude-Lorentz cells (old E from the previous buffers), TF/SF E, sources
@@ -1736,8 +1762,8 @@ cps_status run_op_T(cps_grid *g, const RecOp &o)
 {
     const FieldView<T> f = field_view<T>(g);
     switch (o.kind) {
-    case kOpHBulk: launch_h_bulk<T>(f, g->stream); g->launches++; break;
-    case kOpEBulk: launch_e_bulk<T>(f, g->stream); g->launches++; break;
+    case kOpHBulk: launch_h_bulk<T>(f, pml_view<T>(g), false, g->stream); g->launches++; break;
+    case kOpEBulk: launch_e_bulk<T>(f, pml_view<T>(g), false, g->stream); g->launches++; break;
     case kOpHPml: launch_h_pml<T>(f, pml_view<T>(g), g->stream); g->launches++; break;
     case kOpEPml: launch_e_pml<T>(f, pml_view<T>(g), g->stream); g->launches++; break;
     case kOpDl: launch_dl<T>(f, dl_view<T>(g), g->stream); g->launches++; break;

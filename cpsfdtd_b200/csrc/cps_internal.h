@@ -246,8 +246,10 @@ bool kernel_smem(int bytes, int carveout = -1)
 // ------------------------------------------------------------ launchers
 // Plain path: one kernel per reference routine (kernels_plain.cu, built
 // without FMA contraction so FP64 results follow the reference roundings).
-template <typename T> void launch_h_bulk(const FieldView<T> &f, cudaStream_t s);
-template <typename T> void launch_e_bulk(const FieldView<T> &f, cudaStream_t s);
+// with_pml: the side's CPML routine in the same launch (where no other routine
+// comes between the two at a cell of the slabs)
+template <typename T> void launch_h_bulk(const FieldView<T> &f, const PmlView<T> &p, bool with_pml, cudaStream_t s);
+template <typename T> void launch_e_bulk(const FieldView<T> &f, const PmlView<T> &p, bool with_pml, cudaStream_t s);
 template <typename T> void launch_h_pml(const FieldView<T> &f, const PmlView<T> &p, cudaStream_t s);
 template <typename T> void launch_e_pml(const FieldView<T> &f, const PmlView<T> &p, cudaStream_t s);
 template <typename T> void launch_dl(const FieldView<T> &f, const DlView<T> &d, cudaStream_t s);

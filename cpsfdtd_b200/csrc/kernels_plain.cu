@@ -4,6 +4,8 @@
 // the reference's order, so the FP64 instantiation reproduces the reference
 // arithmetic of BasicFDTD.cpp, CPML.cpp, TF_SF.cpp and the oracle's
 // Drude-Lorentz/gain recursions operation by operation.
+#include <string.h>
+
 #include "batch.h"
 #include "cells.cuh"
 
@@ -13,41 +15,6 @@ namespace {
 
 constexpr int kBY = 8;
 
-// BasicHFieldUpdate, BasicFDTD.cpp:67-84: i,j,k in [0, N-1]
-template <typename T>
-__global__ void __launch_bounds__(32 * kBY) k_h_bulk(FieldView<T> f)
-{
-    const int i = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * kBY + threadIdx.y, k = blockIdx.z;
-    if (i >= f.d.nx || j >= f.d.ny) return;
-    const int64_t g = f.d.idx(i, j, k), sy = f.d.px, sz = f.d.pxy;
-    const int id = f.id[g];
-    const T aH = f.aH[id], bH = f.bH[id];
-    const StretchView<T> &s = f.s;
-    f.Hx[g] = aH * f.Hx[g] - bH * (f.Ez[g + sy] - f.Ez[g]) * s.cHxz[j] + bH * (f.Ey[g + sz] - f.Ey[g]) * s.cHxy[k];
-    f.Hy[g] = aH * f.Hy[g] - bH * (f.Ex[g + sz] - f.Ex[g]) * s.cHyx[k] + bH * (f.Ez[g + 1] - f.Ez[g]) * s.cHyz[i];
-    f.Hz[g] = aH * f.Hz[g] + bH * (f.Ex[g + sy] - f.Ex[g]) * s.cHzx[j] - bH * (f.Ey[g + 1] - f.Ey[g]) * s.cHzy[i];
-}
-
-// BasicEFieldUpdate, BasicFDTD.cpp:25-47: i,j,k in [1, N-1]; ID 4 zeroes E,
-// ID 2 is left to the Drude-Lorentz routine
-template <typename T>
-__global__ void __launch_bounds__(32 * kBY) k_e_bulk(FieldView<T> f)
-{
-    const int i = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * kBY + threadIdx.y, k = blockIdx.z + 1;
-    if (i < 1 || i >= f.d.nx || j < 1 || j >= f.d.ny) return;
-    const int64_t g = f.d.idx(i, j, k), sy = f.d.px, sz = f.d.pxy;
-    const int id = f.id[g];
-    if (id == CPS_ID_PEC) {
-        f.Ex[g] = T(0); f.Ey[g] = T(0); f.Ez[g] = T(0);
-    } else if (id != CPS_ID_DISPERSIVE) {
-        const T aE = f.aE[id], bE = f.bE[id];
-        const StretchView<T> &s = f.s;
-        f.Ex[g] = aE * f.Ex[g] + bE * (f.Hz[g] - f.Hz[g - sy]) * s.cExz[j] - bE * (f.Hy[g] - f.Hy[g - sz]) * s.cExy[k];
-        f.Ey[g] = aE * f.Ey[g] + bE * (f.Hx[g] - f.Hx[g - sz]) * s.cEyx[k] - bE * (f.Hz[g] - f.Hz[g - 1]) * s.cEyz[i];
-        f.Ez[g] = aE * f.Ez[g] + bE * (f.Hy[g] - f.Hy[g - 1]) * s.cEzy[i] - bE * (f.Hx[g] - f.Hx[g - sy]) * s.cEzx[j];
-    }
-}
-
 // psi index of slab-local s at (i,j,k) for axis a (x: [k][j][s], y: [k][s][i], z: [s][j][i])
 __device__ __forceinline__ int64_t psi_index(const Dims &d, int axis, int np, int s, int i, int j, int k)
 {
@@ -56,87 +23,177 @@ __device__ __forceinline__ int64_t psi_index(const Dims &d, int axis, int np, in
     return ((int64_t)s * (d.ny + 1) + j) * d.px + i;
 }
 
-// CPML::UpdateCPMLEFields, one face: CPML.cpp:529-607.  Threads cover
-// (u, v, w) = slab-local index plus the two transverse ranges [1, N-1].
-template <typename T>
-__global__ void k_e_pml_face(FieldView<T> f, PmlView<T> p, int face)
+// slab of index `at` on an axis of n cells (f1 its first face): E slabs are
+// [1, np] and [n-np, n-1] (CPML.cpp:534, 546), H slabs [0, np-1] and [n-np, n-1]
+// (CPML.cpp:614, 626); -1 outside
+__device__ __forceinline__ int slab_of(const int np[6], int f1, int n, int at, bool eside, int &s)
 {
-    const int axis = face >> 1, end = face & 1, np = p.np[face];
+    s = at;
+    if (at < np[f1] + (eside ? 1 : 0)) return f1;
+    s = at - (n - np[f1 + 1]);
+    return s >= 0 ? f1 + 1 : -1;
+}
+
+// one face's psi pair: q <- b q + c d
+template <typename T>
+__device__ __forceinline__ void psi_pair(T *const q[2], int64_t o, T b, T c, T d0, T d1, T &a0, T &a1)
+{
+    a0 = b * q[0][o] + c * d0;
+    a1 = b * q[1][o] + c * d1;
+    q[0][o] = a0;
+    q[1][o] = a1;
+}
+
+// CPML::UpdateCPMLHFields at one cell (CPML.cpp:609-689): the faces in the
+// reference's order x1 x2 y1 y2 z1 z2.  A cell lies in one end of an axis at
+// most, so its corrections are those of the per-face loops in their order.
+template <typename T>
+__device__ __forceinline__ void h_pml_at(const FieldView<T> &f, const PmlView<T> &p, int i, int j, int k, int64_t g,
+                                         int id, T &hx, T &hy, T &hz)
+{
     const Dims &d = f.d;
-    int i, j, k, s;
-    if (axis == 0) {
-        s = blockIdx.x * 32 + threadIdx.x; j = blockIdx.y * kBY + threadIdx.y + 1; k = blockIdx.z + 1;
-        if (s >= np || j >= d.ny) return;
-        i = end == 0 ? s + 1 : d.nx - np + s;
-    } else if (axis == 1) {
-        i = blockIdx.x * 32 + threadIdx.x + 1; s = blockIdx.y * kBY + threadIdx.y; k = blockIdx.z + 1;
-        if (i >= d.nx || s >= np) return;
-        j = end == 0 ? s + 1 : d.ny - np + s;
-    } else {
-        i = blockIdx.x * 32 + threadIdx.x + 1; j = blockIdx.y * kBY + threadIdx.y + 1; s = blockIdx.z;
-        if (i >= d.nx || j >= d.ny) return;
-        k = end == 0 ? s + 1 : d.nz - np + s;
+    int sx, sy, sz;
+    const int fx = slab_of(p.np, kFX1, d.nx, i, false, sx), fy = slab_of(p.np, kFY1, d.ny, j, false, sy);
+    const int fz = slab_of(p.np, kFZ1, d.nz, k, false, sz);
+    if (fx < 0 && fy < 0 && fz < 0) return;
+    const T ch = pml_ch_cell(p, f.bH, id);
+    T a0, a1;
+    if (fx >= 0) {
+        psi_pair(p.qh[fx], psi_index(d, 0, p.np[fx], sx, i, j, k), p.bH[fx][sx], p.cH[fx][sx], f.Ez[g + 1] - f.Ez[g],
+                 f.Ey[g + 1] - f.Ey[g], a0, a1);
+        hy = hy + a0 * ch;
+        hz = hz - a1 * ch;
     }
-    const int cs = end == 0 ? s + 1 : s;  // coefficient index (CPML.cpp:534, 546)
-    const int64_t g = d.idx(i, j, k), q = psi_index(d, axis, np, cs, i, j, k);
-    const T b = p.bE[face][cs], c = p.cE[face][cs], ce = pml_ce_cell(p, f.bE, (int)f.id[g]);
-    T *q0 = p.qe[face][0], *q1 = p.qe[face][1];
-    if (axis == 0) {
-        q0[q] = b * q0[q] + c * (f.Hz[g] - f.Hz[g - 1]);
-        f.Ey[g] = f.Ey[g] - q0[q] * ce;
-        q1[q] = b * q1[q] + c * (f.Hy[g] - f.Hy[g - 1]);
-        f.Ez[g] = f.Ez[g] + q1[q] * ce;
-    } else if (axis == 1) {
-        q0[q] = b * q0[q] + c * (f.Hx[g] - f.Hx[g - d.px]);
-        f.Ez[g] = f.Ez[g] - q0[q] * ce;
-        q1[q] = b * q1[q] + c * (f.Hz[g] - f.Hz[g - d.px]);
-        f.Ex[g] = f.Ex[g] + q1[q] * ce;
-    } else {
-        q0[q] = b * q0[q] + c * (f.Hy[g] - f.Hy[g - d.pxy]);
-        f.Ex[g] = f.Ex[g] - q0[q] * ce;
-        q1[q] = b * q1[q] + c * (f.Hx[g] - f.Hx[g - d.pxy]);
-        f.Ey[g] = f.Ey[g] + q1[q] * ce;
+    if (fy >= 0) {
+        psi_pair(p.qh[fy], psi_index(d, 1, p.np[fy], sy, i, j, k), p.bH[fy][sy], p.cH[fy][sy],
+                 f.Ex[g + d.px] - f.Ex[g], f.Ez[g + d.px] - f.Ez[g], a0, a1);
+        hz = hz - a0 * ch;
+        hx = hx + a1 * ch;
+    }
+    if (fz >= 0) {
+        psi_pair(p.qh[fz], psi_index(d, 2, p.np[fz], sz, i, j, k), p.bH[fz][sz], p.cH[fz][sz],
+                 f.Ey[g + d.pxy] - f.Ey[g], f.Ex[g + d.pxy] - f.Ex[g], a0, a1);
+        hx = hx - a0 * ch;
+        hy = hy + a1 * ch;
     }
 }
 
-// CPML::UpdateCPMLHFields, one face: CPML.cpp:609-689; transverse ranges [0, N-1]
+// CPML::UpdateCPMLEFields at one cell (CPML.cpp:529-607), likewise
 template <typename T>
-__global__ void k_h_pml_face(FieldView<T> f, PmlView<T> p, int face)
+__device__ __forceinline__ void e_pml_at(const FieldView<T> &f, const PmlView<T> &p, int i, int j, int k, int64_t g,
+                                         int id, T &ex, T &ey, T &ez)
 {
-    const int axis = face >> 1, end = face & 1, np = p.np[face];
     const Dims &d = f.d;
-    int i, j, k, s;
-    if (axis == 0) {
-        s = blockIdx.x * 32 + threadIdx.x; j = blockIdx.y * kBY + threadIdx.y; k = blockIdx.z;
-        if (s >= np || j >= d.ny) return;
-        i = end == 0 ? s : d.nx - np + s;
-    } else if (axis == 1) {
-        i = blockIdx.x * 32 + threadIdx.x; s = blockIdx.y * kBY + threadIdx.y; k = blockIdx.z;
-        if (i >= d.nx || s >= np) return;
-        j = end == 0 ? s : d.ny - np + s;
-    } else {
-        i = blockIdx.x * 32 + threadIdx.x; j = blockIdx.y * kBY + threadIdx.y; s = blockIdx.z;
-        if (i >= d.nx || j >= d.ny) return;
-        k = end == 0 ? s : d.nz - np + s;
+    int sx, sy, sz;
+    const int fx = slab_of(p.np, kFX1, d.nx, i, true, sx), fy = slab_of(p.np, kFY1, d.ny, j, true, sy);
+    const int fz = slab_of(p.np, kFZ1, d.nz, k, true, sz);
+    if (fx < 0 && fy < 0 && fz < 0) return;
+    const T ce = pml_ce_cell(p, f.bE, id);
+    T a0, a1;
+    if (fx >= 0) {
+        psi_pair(p.qe[fx], psi_index(d, 0, p.np[fx], sx, i, j, k), p.bE[fx][sx], p.cE[fx][sx], f.Hz[g] - f.Hz[g - 1],
+                 f.Hy[g] - f.Hy[g - 1], a0, a1);
+        ey = ey - a0 * ce;
+        ez = ez + a1 * ce;
     }
-    const int64_t g = d.idx(i, j, k), q = psi_index(d, axis, np, s, i, j, k);
-    const T b = p.bH[face][s], c = p.cH[face][s], ch = pml_ch_cell(p, f.bH, (int)f.id[g]);
-    T *q0 = p.qh[face][0], *q1 = p.qh[face][1];
-    if (axis == 0) {
-        q0[q] = b * q0[q] + c * (f.Ez[g + 1] - f.Ez[g]);
-        f.Hy[g] = f.Hy[g] + q0[q] * ch;
-        q1[q] = b * q1[q] + c * (f.Ey[g + 1] - f.Ey[g]);
-        f.Hz[g] = f.Hz[g] - q1[q] * ch;
-    } else if (axis == 1) {
-        q0[q] = b * q0[q] + c * (f.Ex[g + d.px] - f.Ex[g]);
-        f.Hz[g] = f.Hz[g] - q0[q] * ch;
-        q1[q] = b * q1[q] + c * (f.Ez[g + d.px] - f.Ez[g]);
-        f.Hx[g] = f.Hx[g] + q1[q] * ch;
+    if (fy >= 0) {
+        psi_pair(p.qe[fy], psi_index(d, 1, p.np[fy], sy, i, j, k), p.bE[fy][sy], p.cE[fy][sy],
+                 f.Hx[g] - f.Hx[g - d.px], f.Hz[g] - f.Hz[g - d.px], a0, a1);
+        ez = ez - a0 * ce;
+        ex = ex + a1 * ce;
+    }
+    if (fz >= 0) {
+        psi_pair(p.qe[fz], psi_index(d, 2, p.np[fz], sz, i, j, k), p.bE[fz][sz], p.cE[fz][sz],
+                 f.Hy[g] - f.Hy[g - d.pxy], f.Hx[g] - f.Hx[g - d.pxy], a0, a1);
+        ex = ex - a0 * ce;
+        ey = ey + a1 * ce;
+    }
+}
+
+// BasicHFieldUpdate, BasicFDTD.cpp:67-84: i,j,k in [0, N-1]; PML: the cell's
+// CPML corrections too (steps whose TF/SF-H targets lie outside the slabs, so
+// that nothing comes between the two routines at any cell).  One launch in the
+// place of seven: at 96^3 in FP64 the six face launches took 37 us beside 14 us
+// of bulk update and, with their issue, most of a 114 us step.
+template <typename T, bool PML>
+__global__ void __launch_bounds__(32 * kBY) k_h_bulk(FieldView<T> f, PmlView<T> p)
+{
+    const int i = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * kBY + threadIdx.y, k = blockIdx.z;
+    if (i >= f.d.nx || j >= f.d.ny) return;
+    const int64_t g = f.d.idx(i, j, k), sy = f.d.px, sz = f.d.pxy;
+    const int id = f.id[g];
+    const T aH = f.aH[id], bH = f.bH[id];
+    const StretchView<T> &s = f.s;
+    T hx = aH * f.Hx[g] - bH * (f.Ez[g + sy] - f.Ez[g]) * s.cHxz[j] + bH * (f.Ey[g + sz] - f.Ey[g]) * s.cHxy[k];
+    T hy = aH * f.Hy[g] - bH * (f.Ex[g + sz] - f.Ex[g]) * s.cHyx[k] + bH * (f.Ez[g + 1] - f.Ez[g]) * s.cHyz[i];
+    T hz = aH * f.Hz[g] + bH * (f.Ex[g + sy] - f.Ex[g]) * s.cHzx[j] - bH * (f.Ey[g + 1] - f.Ey[g]) * s.cHzy[i];
+    if (PML) h_pml_at(f, p, i, j, k, g, id, hx, hy, hz);
+    f.Hx[g] = hx;
+    f.Hy[g] = hy;
+    f.Hz[g] = hz;
+}
+
+// BasicEFieldUpdate, BasicFDTD.cpp:25-47: i,j,k in [1, N-1]; ID 4 zeroes E,
+// ID 2 is left to the Drude-Lorentz routine.  PML: the cell's CPML corrections
+// too (steps without dispersive or gain terms whose TF/SF-E targets and sources
+// lie outside the slabs).
+template <typename T, bool PML>
+__global__ void __launch_bounds__(32 * kBY) k_e_bulk(FieldView<T> f, PmlView<T> p)
+{
+    const int i = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * kBY + threadIdx.y, k = blockIdx.z + 1;
+    if (i < 1 || i >= f.d.nx || j < 1 || j >= f.d.ny) return;
+    const int64_t g = f.d.idx(i, j, k), sy = f.d.px, sz = f.d.pxy;
+    const int id = f.id[g];
+    T ex, ey, ez;
+    if (id == CPS_ID_PEC) {
+        ex = T(0); ey = T(0); ez = T(0);
+    } else if (id != CPS_ID_DISPERSIVE) {
+        const T aE = f.aE[id], bE = f.bE[id];
+        const StretchView<T> &s = f.s;
+        ex = aE * f.Ex[g] + bE * (f.Hz[g] - f.Hz[g - sy]) * s.cExz[j] - bE * (f.Hy[g] - f.Hy[g - sz]) * s.cExy[k];
+        ey = aE * f.Ey[g] + bE * (f.Hx[g] - f.Hx[g - sz]) * s.cEyx[k] - bE * (f.Hz[g] - f.Hz[g - 1]) * s.cEyz[i];
+        ez = aE * f.Ez[g] + bE * (f.Hy[g] - f.Hy[g - 1]) * s.cEzy[i] - bE * (f.Hx[g] - f.Hx[g - sy]) * s.cEzx[j];
     } else {
-        q0[q] = b * q0[q] + c * (f.Ey[g + d.pxy] - f.Ey[g]);
-        f.Hx[g] = f.Hx[g] - q0[q] * ch;
-        q1[q] = b * q1[q] + c * (f.Ex[g + d.pxy] - f.Ex[g]);
-        f.Hy[g] = f.Hy[g] + q1[q] * ch;
+        if (!PML) return;
+        ex = f.Ex[g]; ey = f.Ey[g]; ez = f.Ez[g];
+    }
+    if (PML) e_pml_at(f, p, i, j, k, g, id, ex, ey, ez);
+    f.Ex[g] = ex;
+    f.Ey[g] = ey;
+    f.Ez[g] = ez;
+}
+
+// The CPML routine of one side alone, every slab in one launch: the cells of
+// the z slabs, then of the y slabs between them, then of the x slabs between
+// those, a block row of 32 x kBY threads at a time.
+struct SlabBoxes {
+    int n;
+    int start[7];              // first block of each box
+    int i0[6], j0[6], k0[6];   // first cell
+    int ni[6], nj[6], nk[6];   // cells
+};
+
+template <typename T, bool ESIDE>
+__global__ void __launch_bounds__(32 * kBY) k_pml(FieldView<T> f, PmlView<T> p, const __grid_constant__ SlabBoxes B)
+{
+    int b = 0;
+    while (b + 1 < B.n && (int)blockIdx.x >= B.start[b + 1]) ++b;
+    int r = (int)blockIdx.x - B.start[b];
+    const int bx = (B.ni[b] + 31) / 32, by = (B.nj[b] + kBY - 1) / kBY;
+    const int z = r / (bx * by);
+    r -= z * bx * by;
+    const int y = r / bx, u = (r - y * bx) * 32 + (int)threadIdx.x, v = y * kBY + (int)threadIdx.y;
+    if (u >= B.ni[b] || v >= B.nj[b]) return;
+    const int i = B.i0[b] + u, j = B.j0[b] + v, k = B.k0[b] + z;
+    const int64_t g = f.d.idx(i, j, k);
+    if (ESIDE) {
+        T ex = f.Ex[g], ey = f.Ey[g], ez = f.Ez[g];
+        e_pml_at(f, p, i, j, k, g, (int)f.id[g], ex, ey, ez);
+        f.Ex[g] = ex; f.Ey[g] = ey; f.Ez[g] = ez;
+    } else {
+        T hx = f.Hx[g], hy = f.Hy[g], hz = f.Hz[g];
+        h_pml_at(f, p, i, j, k, g, (int)f.id[g], hx, hy, hz);
+        f.Hx[g] = hx; f.Hy[g] = hy; f.Hz[g] = hz;
     }
 }
 
@@ -344,49 +401,65 @@ inline unsigned cdiv(int64_t a, int64_t b) { return (unsigned)((a + b - 1) / b);
 
 }  // namespace
 
+// the slab cells of a side as disjoint boxes
 template <typename T>
-void launch_h_bulk(const FieldView<T> &f, cudaStream_t s)
+static SlabBoxes slab_boxes(const PmlView<T> &p, const Dims &d, bool eside)
 {
-    dim3 grid(cdiv(f.d.nx, 32), cdiv(f.d.ny, kBY), f.d.nz);
-    k_h_bulk<T><<<grid, dim3(32, kBY), 0, s>>>(f);
+    SlabBoxes B;
+    memset(&B, 0, sizeof(B));
+    const int lo = eside ? 1 : 0;  // first updated index
+    const int n[3] = {d.nx, d.ny, d.nz};
+    int a[3], e[3];  // the interior between the slabs, shrunk axis by axis
+    for (int q = 0; q < 3; ++q) { a[q] = lo; e[q] = n[q]; }
+    for (int ax = 2; ax >= 0; --ax)
+        for (int end = 0; end < 2; ++end) {
+            const int np = p.np[2 * ax + end];
+            int b0[3] = {a[0], a[1], a[2]}, b1[3] = {e[0], e[1], e[2]};
+            if (end == 0) {
+                b1[ax] = lo + np;
+                a[ax] = lo + np;
+            } else {
+                b0[ax] = n[ax] - np;
+                e[ax] = n[ax] - np;
+            }
+            if (np <= 0 || b1[0] <= b0[0] || b1[1] <= b0[1] || b1[2] <= b0[2]) continue;
+            const int q = B.n++;
+            B.i0[q] = b0[0]; B.j0[q] = b0[1]; B.k0[q] = b0[2];
+            B.ni[q] = b1[0] - b0[0]; B.nj[q] = b1[1] - b0[1]; B.nk[q] = b1[2] - b0[2];
+            B.start[q + 1] = B.start[q] + (int)(cdiv(B.ni[q], 32) * cdiv(B.nj[q], kBY)) * B.nk[q];
+        }
+    return B;
 }
 
 template <typename T>
-void launch_e_bulk(const FieldView<T> &f, cudaStream_t s)
+void launch_h_bulk(const FieldView<T> &f, const PmlView<T> &p, bool with_pml, cudaStream_t s)
+{
+    dim3 grid(cdiv(f.d.nx, 32), cdiv(f.d.ny, kBY), f.d.nz);
+    if (with_pml) k_h_bulk<T, true><<<grid, dim3(32, kBY), 0, s>>>(f, p);
+    else k_h_bulk<T, false><<<grid, dim3(32, kBY), 0, s>>>(f, p);
+}
+
+template <typename T>
+void launch_e_bulk(const FieldView<T> &f, const PmlView<T> &p, bool with_pml, cudaStream_t s)
 {
     if (f.d.nz < 2) return;
     dim3 grid(cdiv(f.d.nx, 32), cdiv(f.d.ny, kBY), f.d.nz - 1);
-    k_e_bulk<T><<<grid, dim3(32, kBY), 0, s>>>(f);
+    if (with_pml) k_e_bulk<T, true><<<grid, dim3(32, kBY), 0, s>>>(f, p);
+    else k_e_bulk<T, false><<<grid, dim3(32, kBY), 0, s>>>(f, p);
 }
 
 template <typename T>
 void launch_e_pml(const FieldView<T> &f, const PmlView<T> &p, cudaStream_t s)
 {
-    const Dims &d = f.d;
-    for (int face = 0; face < 6; ++face) {  // reference order x1 x2 y1 y2 z1 z2
-        const int np = p.np[face];
-        if (np <= 0) continue;
-        dim3 grid;
-        if (face < 2) grid = dim3(cdiv(np, 32), cdiv(d.ny - 1, kBY), d.nz - 1);
-        else if (face < 4) grid = dim3(cdiv(d.nx - 1, 32), cdiv(np, kBY), d.nz - 1);
-        else grid = dim3(cdiv(d.nx - 1, 32), cdiv(d.ny - 1, kBY), np);
-        k_e_pml_face<T><<<grid, dim3(32, kBY), 0, s>>>(f, p, face);
-    }
+    const SlabBoxes B = slab_boxes(p, f.d, true);
+    if (B.n > 0) k_pml<T, true><<<B.start[B.n], dim3(32, kBY), 0, s>>>(f, p, B);
 }
 
 template <typename T>
 void launch_h_pml(const FieldView<T> &f, const PmlView<T> &p, cudaStream_t s)
 {
-    const Dims &d = f.d;
-    for (int face = 0; face < 6; ++face) {
-        const int np = p.np[face];
-        if (np <= 0) continue;
-        dim3 grid;
-        if (face < 2) grid = dim3(cdiv(np, 32), cdiv(d.ny, kBY), d.nz);
-        else if (face < 4) grid = dim3(cdiv(d.nx, 32), cdiv(np, kBY), d.nz);
-        else grid = dim3(cdiv(d.nx, 32), cdiv(d.ny, kBY), np);
-        k_h_pml_face<T><<<grid, dim3(32, kBY), 0, s>>>(f, p, face);
-    }
+    const SlabBoxes B = slab_boxes(p, f.d, false);
+    if (B.n > 0) k_pml<T, false><<<B.start[B.n], dim3(32, kBY), 0, s>>>(f, p, B);
 }
 
 template <typename T>
@@ -451,8 +524,8 @@ void launch_sources_batch(const BatchGrid<T> *grids, const int2 *ents, int n, in
 }
 
 #define CPS_INSTANTIATE(T)                                                                              \
-    template void launch_h_bulk<T>(const FieldView<T> &, cudaStream_t);                                 \
-    template void launch_e_bulk<T>(const FieldView<T> &, cudaStream_t);                                 \
+    template void launch_h_bulk<T>(const FieldView<T> &, const PmlView<T> &, bool, cudaStream_t);       \
+    template void launch_e_bulk<T>(const FieldView<T> &, const PmlView<T> &, bool, cudaStream_t);       \
     template void launch_h_pml<T>(const FieldView<T> &, const PmlView<T> &, cudaStream_t);              \
     template void launch_e_pml<T>(const FieldView<T> &, const PmlView<T> &, cudaStream_t);              \
     template void launch_dl<T>(const FieldView<T> &, const DlView<T> &, cudaStream_t);                  \
