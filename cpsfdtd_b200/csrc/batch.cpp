@@ -432,9 +432,11 @@ int64_t enqueue_chunk(cps_batch *b, int S)
         });
         launch_inject_batch<T>(G, b->d_inj[0], b->ninj[0], 0, s, st);
         launch_sources_batch<T>(G, b->d_src, b->nsrc, s, st);
-        launch_gather_batch<T>(G, P, b->d_gather, b->ngather, s, S - 1, st);
+        // without a port DFT only the chunk's last sample is kept
+        const bool sample = b->ndft > 0 || s == S - 1;
+        if (sample) launch_gather_batch<T>(G, P, b->d_gather, b->ngather, s, S - 1, st);
         for (int c = 0; c < kNumSweep; ++c) n += b->ntiles[c] > 0;
-        n += (b->ndl > 0) + (b->ninj[0] > 0) + (b->ninj[1] > 0) + (b->nsrc > 0) + (b->ngather > 0);
+        n += (b->ndl > 0) + (b->ninj[0] > 0) + (b->ninj[1] > 0) + (b->nsrc > 0) + (sample && b->ngather > 0);
     }
     launch_dft_batch<T>(G, P, b->d_phasor, b->nphasor, b->d_dft, b->ndft, S, st);
     n += b->ndft > 0 ? 2 : 0;
@@ -483,12 +485,30 @@ cps_status run_chunk(cps_batch *b, int S)
 template <typename T>
 cps_status step_batch_T(cps_batch *b, int nsteps)
 {
-    // rebuild when a member changed since the tables were made
-    if (!b->dirty)
-        for (size_t q = 0; q < b->grids.size(); ++q)
-            if (!(signature(b->grids[q]) == b->sigs[q])) { b->dirty = true; break; }
+    // rebuild when a member changed since the tables were made; a member that
+    // only stepped on its own in between gets its new step number
     cps_status s;
-    if (b->dirty && (s = rebuild_T<T>(b))) return s;
+    std::vector<size_t> moved;
+    if (!b->dirty)
+        for (size_t q = 0; q < b->grids.size(); ++q) {
+            GridSig now = signature(b->grids[q]);
+            if (now == b->sigs[q]) continue;
+            moved.push_back(q);
+            now.step = b->sigs[q].step;
+            if (!(now == b->sigs[q])) { b->dirty = true; break; }
+        }
+    if (b->dirty) {
+        if ((s = rebuild_T<T>(b))) return s;
+        moved.clear();
+    }
+    for (size_t q : moved) {
+        cps_grid *g = b->grids[q];
+        // fold samples left in the rings by one-grid stepping
+        for (PortState &P : g->ports)
+            if (P.fill > 0 && P.nfreq > 0 && (s = flush_dft(g, P))) return s;
+        launch_set_step_batch<T>((BatchGrid<T> *)b->d_grids, (int)q, g->step, b->stream);
+        b->sigs[q].step = g->step;
+    }
     if ((s = sync_grid_streams_in(b))) return s;
     while (nsteps > 0) {
         const int S = std::min(nsteps, kMaxRing);

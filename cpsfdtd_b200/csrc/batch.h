@@ -80,6 +80,9 @@ template <typename T>
 void launch_dl_batch(const BatchGrid<T> *grids, const int4 *blocks, int nblocks, cudaStream_t s);
 template <typename T>
 void launch_advance_batch(BatchGrid<T> *grids, int ngrids, int nsteps, cudaStream_t s);
+// the step number of grid q's descriptor
+template <typename T>
+void launch_set_step_batch(BatchGrid<T> *grids, int q, int64_t n0, cudaStream_t s);
 template <typename T>
 void launch_inject_batch(const BatchGrid<T> *grids, const int4 *blocks, int nblocks, int side, int step_off,
                          cudaStream_t s);

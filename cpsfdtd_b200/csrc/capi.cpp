@@ -1609,17 +1609,22 @@ extern "C" cps_status cps_grid_get_step(const cps_grid *g, int64_t *n)
 }
 
 namespace {
-// grids at or above this size step the fused path as chunks of a one-grid
-// batch: the batch launches their sweeps per grid inside CUDA-graph-replayed
-// chunks and the rest of the step in batched launches, with results equal to
-// the direct launches
-constexpr int64_t kSoloMinCells = 4 << 20;
+// Fused steps run as chunks of a one-grid batch: the batch launches the grid's
+// sweeps inside CUDA-graph-replayed chunks and the rest of the step in batched
+// launches, with results equal to the direct launches.  On a small grid a step
+// is a few microseconds of kernels, far less than its launches take to issue
+// (48^3: 24 us a step launched directly, 12 replayed), on a large one the gaps
+// between them still show (256^3: 2.5 %).  Making the batch's tables takes about
+// the time of 16 direct small steps, so shorter calls on a small grid that has
+// no tables yet are launched directly.
+constexpr int64_t kSoloCells = 4 << 20;
+constexpr int kSoloSteps = 32;
 
-bool solo_eligible(const cps_grid *g)
+bool solo_eligible(const cps_grid *g, int nsteps)
 {
     return g->chunked && g->timing_stride == 0 && g->sweep_mode == 0 && !g->three_on &&
            (g->shape.by == 4 || g->shape.by == 8) && g->d.px >= 64 && g->d.ny >= 8 && g->d.nz >= 2 &&
-           (int64_t)g->d.nx * g->d.ny * g->d.nz >= kSoloMinCells;
+           (g->solo || nsteps >= kSoloSteps || (int64_t)g->d.nx * g->d.ny * g->d.nz >= kSoloCells);
 }
 
 cps_status solo_step(cps_grid *g, int32_t nsteps)
@@ -1635,8 +1640,8 @@ cps_status solo_step(cps_grid *g, int32_t nsteps)
     }
     int32_t rows = 0, planes = 0, pers = 0;
     if ((s = cps_batch_get_tile(g->solo, &rows, &planes, &pers))) return s;
-    if ((rows != g->shape.by || planes != g->shape.kc || pers != 0) &&
-        (s = cps_batch_set_tile(g->solo, g->shape.by, g->shape.kc, 0)))
+    if ((rows != g->shape.by || planes != g->shape.kc || pers != 2) &&
+        (s = cps_batch_set_tile(g->solo, g->shape.by, g->shape.kc, 2)))
         return s;
     batch_use_grid_tiles(g->solo);
     int64_t l0 = 0, l1 = 0;
@@ -1664,7 +1669,7 @@ extern "C" cps_status cps_step(cps_grid *g, int32_t nsteps, int32_t path)
     REQUIRE(path == CPS_PATH_PLAIN || path == CPS_PATH_FUSED || path == CPS_PATH_ONEPASS, CPS_E_INVALID,
             "cps_step: unknown path");
     CK(cudaSetDevice(g->desc.device));
-    if (path == CPS_PATH_FUSED && nsteps > 0 && solo_eligible(g)) return solo_step(g, nsteps);
+    if (path == CPS_PATH_FUSED && nsteps > 0 && solo_eligible(g, nsteps)) return solo_step(g, nsteps);
     return g->fp32 ? step_T<float>(g, nsteps, path) : step_T<double>(g, nsteps, path);
 }
 

@@ -134,6 +134,12 @@ __global__ void k_advance(BatchGrid<T> *grids, int ngrids, int nsteps)
     if (g < ngrids) grids[g].n0 += nsteps;
 }
 
+template <typename T>
+__global__ void k_set_step(BatchGrid<T> *grids, int q, int64_t n0)
+{
+    grids[q].n0 = n0;
+}
+
 inline unsigned cdiv(int64_t a, int64_t b) { return (unsigned)((a + b - 1) / b); }
 
 // set once per kernel and device; false when the attribute could not be set
@@ -259,6 +265,12 @@ void launch_advance_batch(BatchGrid<T> *grids, int ngrids, int nsteps, cudaStrea
 }
 
 template <typename T>
+void launch_set_step_batch(BatchGrid<T> *grids, int q, int64_t n0, cudaStream_t s)
+{
+    k_set_step<T><<<1, 1, 0, s>>>(grids, q, n0);
+}
+
+template <typename T>
 int batch_blocks_per_sm(int by, bool eside, int cls)
 {
     if (by == 4) {
@@ -292,6 +304,7 @@ void batch_kernel_attributes()
                                     cudaStream_t);                                                           \
     template void launch_dl_batch<T>(const BatchGrid<T> *, const int4 *, int, cudaStream_t);                 \
     template void launch_advance_batch<T>(BatchGrid<T> *, int, int, cudaStream_t);                           \
+    template void launch_set_step_batch<T>(BatchGrid<T> *, int, int64_t, cudaStream_t);                      \
     template int batch_blocks_per_sm<T>(int, bool, int);                                              \
     template void batch_kernel_attributes<T>();
 CPS_BATCH_INSTANTIATE(float)
