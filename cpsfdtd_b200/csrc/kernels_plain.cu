@@ -8,6 +8,7 @@
 
 #include "batch.h"
 #include "cells.cuh"
+#include "pdl.cuh"
 
 namespace cps {
 
@@ -118,6 +119,8 @@ __device__ __forceinline__ void e_pml_at(const FieldView<T> &f, const PmlView<T>
 template <typename T, bool PML>
 __global__ void __launch_bounds__(32 * kBY) k_h_bulk(FieldView<T> f, PmlView<T> p)
 {
+    pdl_go();
+    pdl_wait();
     const int i = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * kBY + threadIdx.y, k = blockIdx.z;
     if (i >= f.d.nx || j >= f.d.ny) return;
     const int64_t g = f.d.idx(i, j, k), sy = f.d.px, sz = f.d.pxy;
@@ -140,6 +143,8 @@ __global__ void __launch_bounds__(32 * kBY) k_h_bulk(FieldView<T> f, PmlView<T> 
 template <typename T, bool PML>
 __global__ void __launch_bounds__(32 * kBY) k_e_bulk(FieldView<T> f, PmlView<T> p)
 {
+    pdl_go();
+    pdl_wait();
     const int i = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * kBY + threadIdx.y, k = blockIdx.z + 1;
     if (i < 1 || i >= f.d.nx || j < 1 || j >= f.d.ny) return;
     const int64_t g = f.d.idx(i, j, k), sy = f.d.px, sz = f.d.pxy;
@@ -325,6 +330,8 @@ template <typename T>
 __global__ void k_inject(FieldView<T> f, const InjTarget *tg, int ntarget, const InjContrib *ct,
                          const T *table, int Nt, double n, uint32_t face_mask)
 {
+    pdl_go();
+    pdl_wait();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= ntarget) return;
     inject_target<T>(f, tg[t], ct, table, Nt, n, face_mask);
@@ -342,6 +349,8 @@ __global__ void __launch_bounds__(kInjThreads) k_inject_batch(const BatchGrid<T>
                                                               const int4 *__restrict__ blocks, int side,
                                                               int step_off)
 {
+    pdl_go();
+    pdl_wait();
     const int4 e = blocks[blockIdx.x];
     const int t0 = e.y + (int)threadIdx.x, t1 = t0 + kInjThreads;
     if (t0 >= e.z) return;
@@ -373,6 +382,8 @@ template <typename T>
 __global__ void k_sources_batch(const BatchGrid<T> *__restrict__ grids, const int2 *__restrict__ ents, int n,
                                 int step_off)
 {
+    pdl_go();
+    pdl_wait();
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= n) return;
     const int2 e = ents[q];
@@ -391,6 +402,8 @@ template <typename T>
 __global__ void k_sources(FieldView<T> f, int nsrc, const int64_t *idx, const int32_t *comp,
                           const double *waves, const int32_t *off, const int32_t *len, int n)
 {
+    pdl_go();
+    pdl_wait();
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= nsrc || n < 0 || n >= len[s]) return;
     T *F[6] = {f.Ex, f.Ey, f.Ez, f.Hx, f.Hy, f.Hz};
@@ -435,8 +448,8 @@ template <typename T>
 void launch_h_bulk(const FieldView<T> &f, const PmlView<T> &p, bool with_pml, cudaStream_t s)
 {
     dim3 grid(cdiv(f.d.nx, 32), cdiv(f.d.ny, kBY), f.d.nz);
-    if (with_pml) k_h_bulk<T, true><<<grid, dim3(32, kBY), 0, s>>>(f, p);
-    else k_h_bulk<T, false><<<grid, dim3(32, kBY), 0, s>>>(f, p);
+    if (with_pml) launch_pdl(true, k_h_bulk<T, true>, grid, dim3(32, kBY), 0, s, f, p);
+    else launch_pdl(true, k_h_bulk<T, false>, grid, dim3(32, kBY), 0, s, f, p);
 }
 
 template <typename T>
@@ -444,8 +457,8 @@ void launch_e_bulk(const FieldView<T> &f, const PmlView<T> &p, bool with_pml, cu
 {
     if (f.d.nz < 2) return;
     dim3 grid(cdiv(f.d.nx, 32), cdiv(f.d.ny, kBY), f.d.nz - 1);
-    if (with_pml) k_e_bulk<T, true><<<grid, dim3(32, kBY), 0, s>>>(f, p);
-    else k_e_bulk<T, false><<<grid, dim3(32, kBY), 0, s>>>(f, p);
+    if (with_pml) launch_pdl(true, k_e_bulk<T, true>, grid, dim3(32, kBY), 0, s, f, p);
+    else launch_pdl(true, k_e_bulk<T, false>, grid, dim3(32, kBY), 0, s, f, p);
 }
 
 template <typename T>
@@ -496,7 +509,7 @@ void launch_inject(const FieldView<T> &f, const InjTarget *tg, int ntarget, cons
                    const T *table, int Nt, double n, uint32_t face_mask, cudaStream_t s)
 {
     if (ntarget <= 0) return;
-    k_inject<T><<<cdiv(ntarget, 128), 128, 0, s>>>(f, tg, ntarget, ct, table, Nt, n, face_mask);
+    launch_pdl(true, k_inject<T>, cdiv(ntarget, 128), 128, 0, s, f, tg, ntarget, ct, table, Nt, n, face_mask);
 }
 
 template <typename T>
@@ -505,7 +518,7 @@ void launch_sources(const FieldView<T> &f, int nsrc, const int64_t *idx, const i
                     cudaStream_t s)
 {
     if (nsrc <= 0) return;
-    k_sources<T><<<cdiv(nsrc, 64), 64, 0, s>>>(f, nsrc, idx, comp, waves, wave_off, wave_len, n);
+    launch_pdl(true, k_sources<T>, cdiv(nsrc, 64), 64, 0, s, f, nsrc, idx, comp, waves, wave_off, wave_len, n);
 }
 
 template <typename T>

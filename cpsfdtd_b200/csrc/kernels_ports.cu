@@ -12,6 +12,7 @@
 // scratch table [2][slots][nfreq] (E time, then H time).
 #include "batch.h"
 #include "cells.cuh"
+#include "pdl.cuh"
 
 namespace cps {
 
@@ -21,6 +22,8 @@ namespace {
 template <typename T>
 __global__ void k_gather(FieldView<T> f, GatherBatch b)
 {
+    pdl_go();
+    pdl_wait();
     const GatherDesc &q = b.p[blockIdx.y];
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     const int npts = q.npts;
@@ -167,6 +170,8 @@ template <typename T>
 __global__ void k_gather_batch(const BatchGrid<T> *__restrict__ grids, const BatchPort<T> *__restrict__ ports,
                                const int2 *__restrict__ blocks, int step_off, int last_off)
 {
+    pdl_go();
+    pdl_wait();
     const int2 e = blocks[blockIdx.x];
     const BatchPort<T> &P = ports[e.x];
     const bool last = step_off == last_off;
@@ -286,7 +291,7 @@ template <typename T>
 void launch_port_gather(const FieldView<T> &f, const GatherBatch &b, cudaStream_t s)
 {
     if (b.n <= 0 || b.max_npts <= 0) return;
-    k_gather<T><<<dim3(cdiv(b.max_npts, 256), b.n), 256, 0, s>>>(f, b);
+    launch_pdl(true, k_gather<T>, dim3(cdiv(b.max_npts, 256), b.n), 256, 0, s, f, b);
 }
 
 template <typename T>

@@ -5,6 +5,7 @@
 
 #include <algorithm>
 
+#include "pdl.cuh"
 #include "warp_tiles.cuh"
 
 namespace cps {
@@ -29,11 +30,16 @@ __global__ void __launch_bounds__(32 * BY, GAIN ? 512 / (32 * BY) : 1024 / (32 *
 {
     extern __shared__ __align__(128) unsigned char sm_raw[];
     __shared__ __align__(8) uint64_t full[kStages];
+    pdl_go();
     unsigned char *sm = align_smem(sm_raw);
     const TileXYZ t = box_tile(tb, (int)blockIdx.x);
     const int k0 = max(1, t.bz * kc), k1 = min(t.bz * kc + kc, f.d.nz);
-    if (k0 >= k1) return;
+    if (k0 >= k1) {
+        pdl_wait();
+        return;
+    }
     init_stages(full);
+    pdl_wait();
     uint32_t ctr = 0;
     if (PM == 1 || (PM == 2 && tile_in_pml(p.np, f.d, t.bx * 32, t.by * BY, BY, k0, k1, true)))
         e_tma_body<T, BY, PM != 0, DL, GAIN>(M, f, p, D, G, kc, t, ctr, err, sm, full);
@@ -48,11 +54,16 @@ __global__ void __launch_bounds__(32 * BY) k_h_tma(const __grid_constant__ TmaMa
 {
     extern __shared__ __align__(128) unsigned char sm_raw[];
     __shared__ __align__(8) uint64_t full[kStages];
+    pdl_go();
     unsigned char *sm = align_smem(sm_raw);
     const TileXYZ t = box_tile(tb, (int)blockIdx.x);
     const int k0 = t.bz * kc, k1 = min(k0 + kc, f.d.nz);
-    if (k0 >= k1) return;
+    if (k0 >= k1) {
+        pdl_wait();
+        return;
+    }
     init_stages(full);
+    pdl_wait();
     uint32_t ctr = 0;
     if (PM == 1 || (PM == 2 && tile_in_pml(p.np, f.d, t.bx * 32, t.by * BY, BY, k0, k1, false)))
         h_tma_body<T, BY, PM != 0>(M, f, p, kc, t, ctr, err, sm, full);
@@ -74,12 +85,17 @@ __global__ void __launch_bounds__(32, warp_blocks<T, BY, false>())
 {
     extern __shared__ __align__(128) unsigned char sm_raw[];
     __shared__ __align__(8) uint64_t full[kMaxStages];
+    pdl_go();
     const TileXYZ t = grid_tile((int)blockIdx.x, nbx, nby);
     const int k0 = t.bz * kc, k1 = min(k0 + kc, f.d.nz);
-    if (k0 >= k1) return;
+    if (k0 >= k1) {
+        pdl_wait();
+        return;
+    }
     __shared__ Coef2<T> tab[kTab];
     if (threadIdx.x < kTab) tab[threadIdx.x] = Coef2<T>{f.aH[threadIdx.x], f.bH[threadIdx.x]};
     init_ring(full);
+    pdl_wait();
     Ring R{align_smem(sm_raw), full, warp_ring<T, BY, false>() - 128, 0u, wait_skew(err), err};
     if (PM == 1 || (PM == 2 && tile_in_pml(p.np, f.d, t.bx * 32, t.by * BY, BY, k0, k1, false)))
         h_warp_tile<T, BY, 1, PM != 0>(M, f, p, kc, t, R, tab);
@@ -94,12 +110,17 @@ __global__ void __launch_bounds__(32, warp_blocks<T, BY, GAIN>())
 {
     extern __shared__ __align__(128) unsigned char sm_raw[];
     __shared__ __align__(8) uint64_t full[kMaxStages];
+    pdl_go();
     const TileXYZ t = grid_tile((int)blockIdx.x, nbx, nby);
     const int k0 = max(1, t.bz * kc), k1 = min(t.bz * kc + kc, f.d.nz);
-    if (k0 >= k1) return;
+    if (k0 >= k1) {
+        pdl_wait();
+        return;
+    }
     __shared__ Coef2<T> tab[kTab];
     if (threadIdx.x < kTab) tab[threadIdx.x] = Coef2<T>{f.aE[threadIdx.x], f.bE[threadIdx.x]};
     init_ring(full);
+    pdl_wait();
     Ring R{align_smem(sm_raw), full, warp_ring<T, BY, GAIN>() - 128, 0u, wait_skew(err), err};
     if (PM == 1 || (PM == 2 && tile_in_pml(p.np, f.d, t.bx * 32, t.by * BY, BY, k0, k1, true)))
         e_warp_tile<T, BY, 1, PM != 0, DL, GAIN>(M, f, p, G, kc, t, R, tab);
@@ -204,7 +225,7 @@ int e_tma_launch(const TmaMaps &M, const FieldView<T> &f, const PmlView<T> &p, c
     const int blocks = tb.start[tb.n];
     if (blocks <= 0) return 0;
     if (!set_smem<k_e_tma<T, BY, PM, DL, GAIN>>(L::SMEM)) return 0;
-    k_e_tma<T, BY, PM, DL, GAIN><<<blocks, dim3(32, BY), L::SMEM, s>>>(M, f, p, D, G, kc, tb, err);
+    launch_pdl(!DL, k_e_tma<T, BY, PM, DL, GAIN>, blocks, dim3(32, BY), L::SMEM, s, M, f, p, D, G, kc, tb, err);
     return 1;
 }
 
@@ -216,7 +237,7 @@ int h_tma_launch(const TmaMaps &M, const FieldView<T> &f, const PmlView<T> &p, i
     const int blocks = tb.start[tb.n];
     if (blocks <= 0) return 0;
     if (!set_smem<k_h_tma<T, BY, PM>>(L::SMEM)) return 0;
-    k_h_tma<T, BY, PM><<<blocks, dim3(32, BY), L::SMEM, s>>>(M, f, p, kc, tb, err);
+    launch_pdl(true, k_h_tma<T, BY, PM>, blocks, dim3(32, BY), L::SMEM, s, M, f, p, kc, tb, err);
     return 1;
 }
 
@@ -227,7 +248,7 @@ int h_warp_launch(const SweepMaps &M, const FieldView<T> &f, const PmlView<T> &p
     constexpr int smem = warp_ring<T, BY, false>();
     const int nbx = (int)cdiv(f.d.nx, 32), nby = (int)cdiv(f.d.ny, BY), nbz = (int)cdiv(f.d.nz, kc);
     if (!set_smem<k_h_warp<T, BY, PM>>(smem)) return 0;
-    k_h_warp<T, BY, PM><<<nbx * nby * nbz, 32, smem, s>>>(M, f, p, kc, nbx, nby, err);
+    launch_pdl(true, k_h_warp<T, BY, PM>, nbx * nby * nbz, 32, smem, s, M, f, p, kc, nbx, nby, err);
     return 1;
 }
 
@@ -239,7 +260,7 @@ int e_warp_launch(const SweepMaps &M, const FieldView<T> &f, const PmlView<T> &p
     constexpr int smem = warp_ring<T, BY, GAIN>();
     const int nbx = (int)cdiv(f.d.nx, 32), nby = (int)cdiv(f.d.ny, BY), nbz = (int)cdiv(f.d.nz, kc);
     if (!set_smem<k_e_warp<T, BY, PM, DL, GAIN>>(smem)) return 0;
-    k_e_warp<T, BY, PM, DL, GAIN><<<nbx * nby * nbz, 32, smem, s>>>(M, f, p, G, kc, nbx, nby, err);
+    launch_pdl(!DL, k_e_warp<T, BY, PM, DL, GAIN>, nbx * nby * nbz, 32, smem, s, M, f, p, G, kc, nbx, nby, err);
     return 1;
 }
 

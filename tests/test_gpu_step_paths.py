@@ -1,0 +1,112 @@
+"""One step's work in different launches: the plain path against its routines
+called one by one (the CPML boxes of a side as one launch, or as part of the
+bulk update's where no injection or source lies in a slab), and small grids'
+fused steps as replayed graph chunks, in ragged pieces, against one launch
+after another.  The same operations in the same order on each cell, so both
+are equal bit for bit."""
+import numpy as np
+import pytest
+
+from conftest import rel_l2
+from cpsfdtd_b200 import decks
+
+pytestmark = pytest.mark.gpu
+
+
+def _tfsf_deck(inset):
+    """TF/SF box `inset` cells inside, CPML of unequal depths, a source."""
+    nx, ny, nz, d = 37, 29, 33, 5e-9
+    dk = decks.Deck(nx, ny, nz, d, d, d)
+    dk.media = [(1.0, 1.0, 0.0, 0.0), (2.25, 1.0, 0.0, 0.0), (1.0, 1.0, 0.0, 0.0)]
+    ids = np.zeros(dk.shape3, dtype=np.uint8)
+    ids[12:20, 10:16, 11:19] = 1
+    dk.ids = ids
+    dk.pml = decks.pml_params(1)
+    dk.pml["npml"] = [5, 5, 3, 3, 4, 4]
+    dk.tfsf = {"lambda": 550e-9, "dlambda": decks.dlambda_for_tau(550e-9, 2e-15), "w0": 100e-9, "z0_deck": 0.0,
+               "xs": (nx / 2 + 0.5) * d, "ys": (ny / 2 + 0.5) * d, "zs": 0.0, "k0": nz // 2, "theta": 30.0,
+               "phi": 45.0, "E0": 1.0, "psi": 0.0, "n6": [inset] * 6, "Nt": 400, "cwmode": 0}
+    return dk
+
+
+def _sourced(dk, at):
+    dk.sources = [(decks.COMP["Ez"], *at, decks.gaussian_sine(400, dk.dt, 600e-9, 5e-16, 7e-16)),
+                  (decks.COMP["Ex"], 15, 14, 16, decks.gaussian_sine(30, dk.dt, 500e-9, 4e-16, 5e-16))]
+    return dk
+    return dk
+
+
+_DECKS = {
+    "clear": lambda: _sourced(_tfsf_deck(9), (18, 12, 16)),
+    "box-meets-slab": lambda: _sourced(_tfsf_deck(5), (18, 12, 16)),
+    "source-in-slab": lambda: _sourced(_tfsf_deck(9), (3, 12, 16)),
+    "source-at-slab-edge": lambda: _sourced(_tfsf_deck(9), (18, 12, 28)),
+    "dispersive": lambda: decks.config2(n=41, steps=1, nfreq=3),
+    "laser": lambda: decks.config4_member(40, 33, 36, seed=3, steps=1, nfreq=2),
+}
+
+
+def _state(g):
+    return [g.field(c) for c in range(6)] + [g.port_last(p) for p in range(len(g.ports))] + [
+        g.port_dft(p, raw=True).copy() for p in range(len(g.ports)) if g.ports[p][2] > 0]
+
+
+def _same(a, b):
+    assert np.abs(a[2]).max() > 0
+    for q, (x, y) in enumerate(zip(a, b)):
+        assert np.array_equal(x, y), (q, rel_l2(x, y))
+
+
+def _noise(g, dk, seed):
+    rng = np.random.Generator(np.random.PCG64(seed))
+    for c in range(6):
+        g.set_field(c, rng.standard_normal(dk.shape3) * (1.0 if c < 3 else 1.0 / 376.7))
+
+
+@pytest.mark.parametrize("name", list(_DECKS))
+@pytest.mark.parametrize("prec", [0, 1], ids=["fp64", "fp32"])
+def test_plain_step_equals_its_routines(name, prec):
+    import cpsfdtd_b200 as cps
+    dk = _DECKS[name]()
+    a, b = cps.Grid.from_deck(dk, prec), cps.Grid.from_deck(dk, prec)
+    for g in (a, b):
+        _noise(g, dk, 5)
+    a.step(12, cps.PLAIN)
+    b.set_record(False)
+    n0 = b.get_step()
+    for n in range(n0, n0 + 12):
+        b.op("h_bulk")
+        if dk.tfsf:
+            b.op("tfsf_h", n, 0x3F)
+        b.op("h_pml")
+        b.op("e_bulk")
+        if dk.dl:
+            b.op("dl")
+        if dk.gain:
+            for q in ("gain_polarization", "gain_efield", "gain_populations"):
+                b.op(q)
+        if dk.tfsf:
+            b.op("tfsf_e", n, 0x3F)
+        if dk.sources:
+            b.op("sources", n)
+        b.op("e_pml")
+        for p in range(len(b.ports)):
+            b.op("port_sample", p, n)
+    _same(_state(a), _state(b))
+
+
+@pytest.mark.parametrize("name", list(_DECKS))
+@pytest.mark.parametrize("prec", [0, 1], ids=["fp64", "fp32"])
+def test_small_grids_chunks_equal_single_launches(name, prec):
+    import cpsfdtd_b200 as cps
+    dk = _DECKS[name]()
+    a, b = cps.Grid.from_deck(dk, prec), cps.Grid.from_deck(dk, prec)
+    b.set_chunked(False)
+    for g in (a, b):
+        _noise(g, dk, 6)
+        g.step(5, cps.FUSED)    # single launches on both
+        g.step(100, cps.FUSED)  # chunks of 64 and 36
+        g.step(1, cps.FUSED)
+        g.step(2, cps.PLAIN)    # the step number moves outside the chunks
+        g.step(67, cps.FUSED)
+    _same(_state(a), _state(b))
