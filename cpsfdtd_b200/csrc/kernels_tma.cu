@@ -221,7 +221,7 @@ template <typename T, int BY, int PM, bool DL, bool GAIN>
 int e_tma_launch(const TmaMaps &M, const FieldView<T> &f, const PmlView<T> &p, const DlView<T> &D,
                  const GainView<T> &G, int kc, const TileBoxes &tb, int *err, cudaStream_t s)
 {
-    using L = StageLayout<T, BY, GAIN && sizeof(T) == 4>;
+    using L = ELayout<T, BY, GAIN>;
     const int blocks = tb.start[tb.n];
     if (blocks <= 0) return 0;
     if (!set_smem<k_e_tma<T, BY, PM, DL, GAIN>>(L::SMEM)) return 0;
@@ -269,7 +269,7 @@ template <typename T, int BY>
 void attrs_by()
 {
     constexpr int S = warp_ring<T, BY, false>(), SB = StageLayout<T, BY>::SMEM;
-    constexpr int SG = StageLayout<T, BY, sizeof(T) == 4>::SMEM;
+    constexpr int SG = ELayout<T, BY, true>::SMEM;
     if constexpr (sizeof(T) == 4) {
         set_smem<k_h_warp<T, BY, 0>>(S);
         set_smem<k_h_warp<T, BY, 2>>(S);

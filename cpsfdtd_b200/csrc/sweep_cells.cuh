@@ -388,6 +388,117 @@ __device__ __forceinline__ void gain_warp(const GainView<T> &G, const Dims &d, i
     ex = E[0]; ey = E[1]; ez = E[2];
 }
 
+// ---- FP64 gain in the block-tile E sweep.  What bounded it was latency at 16
+// warps per SM: the 16 words of a cell (Pa Pa1 Pb Pb1 x3, N0..N3) were asked
+// for after the list look-up and right before their use, the CPML body spilled
+// to a memory that L1, what the stages leave of it, does not hold, and fourteen
+// divisions a cell ran one after the other.  Now a row segment's list offset
+// and gain mask come a plane ahead, the words are asked for at the top of the
+// plane and used at its end, the psi words of the next plane go to shared slots
+// of their own lane (8-byte asynchronous copies: no registers, no barrier) and
+// the eleven divisions by constants are three operations each.  176^3 laser:
+// CPML tiles 309 -> 222 us, interior 236 -> 187 us, 76 % of the copy bandwidth.
+// (The gain words through shared slots too: 249 and 215 us, the 8-byte copies
+// then fill the load-store queue.)
+constexpr int kFetchSlots = 6;  // psi words per lane
+
+__device__ __forceinline__ void cp_async8(void *dst, const void *src)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// psi_load_e into slots
+__device__ __forceinline__ void psi_fetch_e(const PmlView<double> &p, const Dims &d, const ColPml<double> &c, int i,
+                                            int j, int k, double *slot)
+{
+    if (c.fx >= 0) {
+        const int64_t q = ((int64_t)k * (d.ny + 1) + j) * psi_xw(p.np[c.fx]) + c.sxl;
+        cp_async8(slot, p.qe[c.fx][0] + q); cp_async8(slot + 32, p.qe[c.fx][1] + q);
+    }
+    if (c.fy >= 0) {
+        const int64_t q = ((int64_t)k * (p.np[c.fy] + 1) + c.syl) * d.px + i;
+        cp_async8(slot + 64, p.qe[c.fy][0] + q); cp_async8(slot + 96, p.qe[c.fy][1] + q);
+    }
+    int fz = -1, szl = 0;
+    if (k <= p.np[kFZ1]) { fz = kFZ1; szl = k; }
+    else if (k >= d.nz - p.np[kFZ2]) { fz = kFZ2; szl = k - (d.nz - p.np[kFZ2]); }
+    if (fz >= 0) {
+        const int64_t q = ((int64_t)szl * (d.ny + 1) + j) * d.px + i;
+        cp_async8(slot + 128, p.qe[fz][0] + q); cp_async8(slot + 160, p.qe[fz][1] + q);
+    }
+}
+
+
+struct GainRegs64 {
+    double a[6], b[6];  // Pa Pa1, Pb Pb1
+    Pops<double> N;
+};
+// m: list offset and gain mask of the lane's row segment; the returned state
+// pointer is null on a lane without a gain cell
+__device__ __forceinline__ double *gain_fetch64(const GainView<double> &G, uint2 m, GainRegs64 &r)
+{
+    if (!((m.y >> (threadIdx.x & 31u)) & 1u)) return nullptr;
+    using L = GainSite64;
+    double *st = G.state + gain_base_index((int64_t)m.x + __popc(m.y & lanemask_lt()), kG64Words);
+#pragma unroll
+    for (int w = 0; w < 6; ++w) { r.a[w] = st[(L::PA + w) * kGainGroup]; r.b[w] = st[(L::PB + w) * kGainGroup]; }
+    gain_load_n<double>(st, kGainGroup, r.N);
+    return st;
+}
+
+// a / b by b's reciprocal r = 1 / b (rounded): a quotient to an ulp or two and
+// one Newton correction with its exact remainder (Markstein, IBM J. Res. Dev.
+// 34, 1990), three operations against the dozen and the branch of a division
+__device__ __forceinline__ double div_by(double a, double b, double r)
+{
+    const double q = a * r;
+    return __fma_rn(__fma_rn(-q, b, a), r, q);
+}
+
+// gain_n_update<double> with the constant divisors' reciprocals from the host
+__device__ __forceinline__ void gain_n64(const GainCoef &G, Pops<double> &P, const double E[3], const double E1[3],
+                                         const double Pa[3], const double Pa1[3], const double Pa2[3],
+                                         const double Pb[3], const double Pb2[3])
+{
+    double *N = P.N;
+    const double sb = E1[0] * (Pb[0] - Pb2[0]) + E1[1] * (Pb[1] - Pb2[1]) + E1[2] * (Pb[2] - Pb2[2]);
+    const double sa = E1[0] * (Pa[0] - Pa2[0]) + E1[1] * (Pa[1] - Pa2[1]) + E1[2] * (Pa[2] - Pa2[2]);
+    const double s2 = (E[0] + E1[0]) * (Pa[0] - Pa2[0]) + (E[1] + E1[1]) * (Pa[1] - Pa1[1]) +
+                      (E[2] + E1[2]) * (Pa[2] - Pa2[2]);
+    const double N0old = N[0];
+    N[3] = G.t30t32dt / (G.t30t32_2 + G.t30dt * (1 - N[2]) + G.t32dt * (1 - N[0])) *
+           (N[3] * (div_by(N[0] - 1, G.t30, G.r_t30) + div_by(N[2] - 1, G.t32, G.r_t32) + G.dt_2) +
+            div_by(sb, G.homega_bdt, G.r_hwb));
+    N[3] = N[3] + G.pump_dt * N0old;
+    N[1] = G.t10t21dt / (G.t10t21_2 + G.t10dt * N[2] + G.t21dt * (1 - N[0])) *
+           (N[1] * (div_by(N[0] - 1, G.t10, G.r_t10) - div_by(N[2], G.t21, G.r_t21) + G.dt_2) +
+            div_by(N[2], G.t21_2, G.r_t21_2) - div_by(sa, G.homega_adt, G.r_hwa));
+    N[2] = G.t32t21dt / (G.t32t21_2 + G.t21dt * N[3] + G.t32dt * (1 - N[1])) *
+           (N[2] * (div_by(N[1] - 1, G.t21, G.r_t21) - div_by(N[3], G.t32, G.r_t32) + G.dt_2) +
+            div_by(N[3], G.t32_2, G.r_t32_2) + div_by(s2, G.homega_adt, G.r_hwa));
+    N[0] = 2.0 - N[1] - N[2] - N[3];
+}
+
+// P -> E -> N at a gain cell from its words (gain_warp's arithmetic)
+__device__ __forceinline__ void gain_apply64(const GainView<double> &G, double *st, GainRegs64 &r, double &ex,
+                                             double &ey, double &ez)
+{
+    using L = GainSite64;
+    constexpr int64_t sc = kGainGroup;
+    double E[3] = {ex, ey, ez};
+    const double E1[3] = {ex, ey, ez};
+    double Pa2[3], Pb2[3];
+    gain_p_update<double>(G.c, r.N, E, r.a, r.a + 3, Pa2, r.b, r.b + 3, Pb2);
+#pragma unroll
+    for (int q = 0; q < 3; ++q) E[q] = gain_e_corr<double>(G.c, E[q], r.a[q], r.a[3 + q], r.b[q], r.b[3 + q]);
+    gain_n64(G.c, r.N, E, E1, r.a, r.a + 3, Pa2, r.b, Pb2);
+#pragma unroll
+    for (int q = 0; q < 6; ++q) { st[(L::PA + q) * sc] = r.a[q]; st[(L::PB + q) * sc] = r.b[q]; }
+    gain_store_n<double>(st, sc, r.N);
+    ex = E[0]; ey = E[1]; ez = E[2];
+}
 
 // ---- FP32 gain on the segment-dense layout: the 15 persistent words of the
 // cell at device index g are at gain_dense_index(g) + 32 w, for every cell of

@@ -61,9 +61,28 @@ struct StageLayout {
     static constexpr int SMEM = NS * STAGE_B + 128;
 };
 
-// the stage layout of an E sweep (FP32 with gain stages the gain words)
+// the stage layout of an E sweep (FP32 with gain stages the gain words; FP64
+// with gain keeps slots for each lane's psi words behind the stages)
 template <typename T, int BY, bool GAIN>
-using ELayout = StageLayout<T, BY, GAIN && sizeof(T) == 4>;
+struct ELayout : StageLayout<T, BY, GAIN && sizeof(T) == 4> {
+    using S = StageLayout<T, BY, GAIN && sizeof(T) == 4>;
+    static constexpr int WORDS_OFF = S::NS * S::STAGE_B;
+    static constexpr int SMEM = S::SMEM + (GAIN && sizeof(T) == 8 ? kFetchSlots * 32 * BY * 8 : 0);
+};
+
+// the coefficients (a, b) of the first kTab media, in shared memory
+constexpr int kTab = 16;
+template <typename T>
+struct alignas(2 * sizeof(T)) Coef2 {
+    T a, b;
+};
+// the coefficients of medium id: the table's, or from the arrays past it
+template <typename T>
+__device__ __forceinline__ Coef2<T> coef_of(int id, const Coef2<T> *tab, const T *ga, const T *gb)
+{
+    if (id < kTab) return tab[id];
+    return Coef2<T>{__ldg(&ga[id]), __ldg(&gb[id])};
+}
 
 struct TileXYZ {
     int bx, by, bz;  // tile index along x (32 columns), y (BY rows), z (kc planes)
@@ -163,13 +182,18 @@ __device__ __forceinline__ bool e_tma_body(const TmaMaps &M, const FieldView<T> 
 {
     // FP32 gain: the tile's gain words travel with its fields in every stage
     constexpr bool GST = GAIN && sizeof(T) == 4;
-    using L = StageLayout<T, BY, GST>;
+    constexpr bool G64 = GAIN && sizeof(T) == 8;
+    using L = ELayout<T, BY, GAIN>;
     const Dims d = f.d;
     const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * 32 + tx;
     const int x0 = t.bx * 32, y0 = t.by * BY;
     const int i = x0 + tx, j = y0 + ty;
     const int k0 = max(1, t.bz * kc), k1 = min(t.bz * kc + kc, d.nz);
     if (k0 >= k1) return true;  // whole block
+    // looked up per cell and plane: from global memory each plane would wait
+    // for it, L1 being what the stages leave of it
+    __shared__ Coef2<T> tab[kTab];
+    if (tid < kTab) tab[tid] = Coef2<T>{f.aE[tid], f.bE[tid]};  // seen past the first wait's barrier
     const bool rowok = j >= 1 && j < d.ny;
     const bool act = rowok && i >= 1 && i < d.nx;
     const uint32_t c0 = ctr;
@@ -199,14 +223,36 @@ __device__ __forceinline__ bool e_tma_body(const TmaMaps &M, const FieldView<T> 
         hym = __ldg(&f.Hy[gm]);
     }
     // psi two planes ahead: qc (plane k), qn (k+1), loads for k+2 issued at plane k
+    // (one plane ahead, in shared slots, beside an FP64 cell's gain words)
     PsiRegs<T> qc{}, qn{}, qnn{};
-    if (PML && act) {
+    if (PML && act && !G64) {
         psi_load_e(p, d, pc, i, j, k0, qc);
         if (k0 + 1 < k1) psi_load_e(p, d, pc, i, j, k0 + 1, qn);
     }
+    T cExy = sv.cExy[k0], cEyx = sv.cEyx[k0];
     const int hr = (ty + 1) * L::HW + tx + 4, orow = ty * L::OW + tx;
+    // FP64 gain: the row segment's list offset and mask (rm) a plane ahead
+    double *slot = nullptr, *gst = nullptr;
+    const uint2 *rp = nullptr;
+    uint2 rm = make_uint2(0, 0);
+    const int64_t rstep = (int64_t)(d.ny + 1) * (d.px >> 5);
+    if constexpr (G64) {
+        slot = (double *)(sm + L::WORDS_OFF) + ty * (kFetchSlots * 32) + tx;
+        if (rowok) {
+            rp = G.segm + ((int64_t)k0 * (d.ny + 1) + j) * (d.px >> 5) + t.bx;
+            rm = __ldg(rp);
+        }
+        if (PML && act) psi_fetch_e(p, d, pc, i, j, k0, slot);
+    }
     for (int k = k0, it = 0; k < k1; ++k, ++it) {
-        if (PML && act && k + 2 < k1) psi_load_e(p, d, pc, i, j, k + 2, qnn);
+        if (PML && act && !G64 && k + 2 < k1) psi_load_e(p, d, pc, i, j, k + 2, qnn);
+        GainRegs64 gr;
+        if constexpr (G64) {
+            gst = gain_fetch64(G, rm, gr);
+            if (rowok && k + 1 < k1) rm = __ldg(rp += rstep);
+        }
+        const int kn = min(k + 1, k1 - 1);
+        const T nExy = sv.cExy[kn], nEyx = sv.cEyx[kn];  // the next plane's
         const uint32_t q = c0 + (uint32_t)it;
         const int s = (int)(q % L::NS);
         const bool ok = wait_stage(&full[s], (q / L::NS) & 1u);
@@ -215,6 +261,7 @@ __device__ __forceinline__ bool e_tma_body(const TmaMaps &M, const FieldView<T> 
                 atomicExch(err, 1);
                 drain_stages<L::NS>(full, c0, it + 1, min(it + L::NS - 1, npl - 1));
             }
+            if (G64) cp_async_wait_all();
             return false;
         }
         const unsigned char *b = sm + s * L::STAGE_B;
@@ -228,14 +275,13 @@ __device__ __forceinline__ bool e_tma_body(const TmaMaps &M, const FieldView<T> 
         const T dHy_k = hy - hym, dHx_k = hx - hxm;
         T ex = ext[orow], ey = eyt[orow], ez = ezt[orow];
         const int id = idt[orow];
-        const T cExy = sv.cExy[k], cEyx = sv.cEyx[k];
+        Coef2<T> m = coef_of(id, tab, f.aE, f.bE);
         if (id == CPS_ID_PEC) {
             ex = T(0); ey = T(0); ez = T(0);
         } else if (id != CPS_ID_DISPERSIVE) {
-            const T aE = __ldg(&f.aE[id]), bE = __ldg(&f.bE[id]);
-            ex = yee(aE, ex, bE, dHz_j, cExz, dHy_k, cExy);
-            ey = yee(aE, ey, bE, dHx_k, cEyx, dHz_i, cEyz);
-            ez = yee(aE, ez, bE, dHy_i, cEzy, dHx_j, cEzx);
+            ex = yee(m.a, ex, m.b, dHz_j, cExz, dHy_k, cExy);
+            ey = yee(m.a, ey, m.b, dHx_k, cEyx, dHz_i, cEyz);
+            ez = yee(m.a, ez, m.b, dHy_i, cEzy, dHx_j, cEzx);
         }
         if constexpr (GST) {
             // the gain list holds interior cells only (act), with the gain ID
@@ -244,20 +290,32 @@ __device__ __forceinline__ bool e_tma_body(const TmaMaps &M, const FieldView<T> 
                 gain_staged32((const float *)(b + L::GAIN_OFF) + ty * kGainPersist * 32 + tx, r);
                 gain_apply32(G, d.idx(i, j, k), r, ex, ey, ez);
             }
-        } else if (GAIN && rowok) {
-            gain_warp(G, d, j, k, t.bx, act, id, ex, ey, ez);
+        } else if constexpr (G64) {
+            if (rowok) {
+                if (gst) gain_apply64(G, gst, gr, ex, ey, ez);
+                if (PML) {
+                    cp_async_wait_all();
+                    const double *qs = slot;
+                    qc.x0 = qs[0]; qc.x1 = qs[32]; qc.y0 = qs[64]; qc.y1 = qs[96]; qc.z0 = qs[128]; qc.z1 = qs[160];
+                }
+            }
         }
         // ID-2 cells are left untouched here: the Drude-Lorentz cell kernel
         // updates them (ADE, then CPML, the reference order) beside the sweep
         if (act && !(DL && id == CPS_ID_DISPERSIVE)) {
-            if (PML) pml_e_cell_pre(p, d, pc, pml_ce_cell(p, f.bE, id), i, j, k, qc, dHz_i, dHy_i, dHx_j, dHz_j, dHy_k, dHx_k, ex, ey, ez);
+            if (PML) pml_e_cell_pre(p, d, pc, p.literal ? p.cpmlE : id == CPS_ID_DISPERSIVE ? p.ce_disp : m.b,
+                                    i, j, k, qc, dHz_i, dHy_i, dHx_j, dHz_j, dHy_k, dHx_k, ex, ey, ez);
             const int64_t g = d.idx(i, j, k);
             f.Ex[g] = ex; f.Ey[g] = ey; f.Ez[g] = ez;
         }
         hxm = hx; hym = hy;
         qc = qn;
         qn = qnn;
+        cExy = nExy; cEyx = nEyx;
         __syncthreads();
+        if constexpr (G64) {
+            if (PML && act && k + 1 < k1) psi_fetch_e(p, d, pc, i, j, k + 1, slot);
+        }
         if (tid == 0 && k + L::NS < k1) issue(it + L::NS, k + L::NS);
     }
     ctr = c0 + (uint32_t)(k1 - k0);
@@ -277,6 +335,8 @@ __device__ __forceinline__ bool h_tma_body(const TmaMaps &M, const FieldView<T> 
     const int i = x0 + tx, j = y0 + ty;
     const int k0 = t.bz * kc, k1 = min(k0 + kc, d.nz);
     if (k0 >= k1) return true;
+    __shared__ Coef2<T> tab[kTab];
+    if (tid < kTab) tab[tid] = Coef2<T>{f.aH[tid], f.bH[tid]};  // seen past the first wait's barrier
     const bool rowok = j < d.ny;
     const bool act = rowok && i < d.nx;
     const uint32_t c0 = ctr;
@@ -315,6 +375,7 @@ __device__ __forceinline__ bool h_tma_body(const TmaMaps &M, const FieldView<T> 
     // register slots (the loop is unrolled by two, so the slots are never copied)
     PsiRegs<T> qA{}, qB{};
     if (PML && act) psi_load_h(p, d, pc, i, j, k0, qA);
+    T cHxy = sv.cHxy[k0], cHyx = sv.cHyx[k0];
     for (int kb = k0, itb = 0; kb < k1; kb += 2, itb += 2) {
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
@@ -322,6 +383,8 @@ __device__ __forceinline__ bool h_tma_body(const TmaMaps &M, const FieldView<T> 
             if (k >= k1) break;
             PsiRegs<T> &qc = u == 0 ? qA : qB, &qn = u == 0 ? qB : qA;
             if (PML && act && k + 1 < k1) psi_load_h(p, d, pc, i, j, k + 1, qn);
+            const int kn = min(k + 1, k1 - 1);
+            const T nHxy = sv.cHxy[kn], nHyx = sv.cHyx[kn];  // the next plane's
             const uint32_t q = c0 + (uint32_t)it, qn1 = q + 1u;
             const int s = (int)(q % kStages), sn = (int)(qn1 % kStages);
             const bool ok = wait_stage(&full[sn], (qn1 / kStages) & 1u);
@@ -343,18 +406,19 @@ __device__ __forceinline__ bool h_tma_body(const TmaMaps &M, const FieldView<T> 
             const T dEx_j = ext[er + L::HW] - ex, dEy_i = eyt[er + 1] - ey;
             const T dEx_k = exk - ex, dEy_k = eyk - ey;
             const int id = idt[orow];
-            const T aH = __ldg(&f.aH[id]), bH = __ldg(&f.bH[id]);
-            T hx = yee_n(aH, hxt[orow], bH, dEz_j, cHxz, dEy_k, sv.cHxy[k]);
-            T hy = yee_n(aH, hyt[orow], bH, dEx_k, sv.cHyx[k], dEz_i, cHyz);
-            T hz = yee_z(aH, hzt[orow], bH, dEx_j, cHzx, dEy_i, cHzy);
+            const Coef2<T> m = coef_of(id, tab, f.aH, f.bH);
+            T hx = yee_n(m.a, hxt[orow], m.b, dEz_j, cHxz, dEy_k, cHxy);
+            T hy = yee_n(m.a, hyt[orow], m.b, dEx_k, cHyx, dEz_i, cHyz);
+            T hz = yee_z(m.a, hzt[orow], m.b, dEx_j, cHzx, dEy_i, cHzy);
             if (act) {
                 if (PML)
-                    pml_h_cell_pre(p, d, pc, pml_ch_cell(p, f.bH, id), i, j, k, qc, dEz_i, dEy_i, dEx_j, dEz_j, dEy_k,
+                    pml_h_cell_pre(p, d, pc, p.literal ? p.cpmlH : m.b, i, j, k, qc, dEz_i, dEy_i, dEx_j, dEz_j, dEy_k,
                                    dEx_k, hx, hy, hz);
                 const int64_t g = d.idx(i, j, k);
                 f.Hx[g] = hx; f.Hy[g] = hy; f.Hz[g] = hz;
             }
             ex = exk; ey = eyk;
+            cHxy = nHxy; cHyx = nHyx;
             __syncthreads();
             if (tid == 0 && k + kStages <= k1) issue(it + kStages, k + kStages);
         }

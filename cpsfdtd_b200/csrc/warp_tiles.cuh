@@ -348,13 +348,6 @@ __device__ __forceinline__ unsigned vec_ids(const uint8_t *p)
     return *reinterpret_cast<const uint16_t *>(p);
 }
 
-// the coefficients (a, b) of the first kTab media, in shared memory
-constexpr int kTab = 16;
-template <typename T>
-struct alignas(2 * sizeof(T)) Coef2 {
-    T a, b;
-};
-
 // (a, b) of the media of a vector's cells; one look-up when the whole warp
 // holds one medium, which the return value says (its ID, -1 mixed)
 template <typename T>
