@@ -61,68 +61,95 @@ __global__ void k_phasors(const double *omega, int nfreq, int nslots, int64_t n_
     phasor_entry(omega, nfreq, nslots, n_first, dt, q, tab);
 }
 
-// Contraction of one flush: a block of 256 threads covers PT points x FT
-// frequencies of one component (64 x 64, or 128 x 32 for ports with at most
-// 32 frequencies); thread (tp, tf), tp < PT/4, tf < FT/4, owns points
-// p0 + (PT/4)a + tp (a = 0..3) at frequencies f0 + 4tf + b (b = 0..3), so
-// neighbouring lanes touch neighbouring points in shared memory and in the
-// accumulators.  The block's samples [slots][PT] and phasors [slots][FT] are
-// staged in shared memory; each thread loads its 16 FP64 accumulator pairs,
-// adds the samples one slot at a time (acc_re += s cos, acc_im -= s sin,
-// FP64 fused multiply-adds) and stores them back.  Every accumulator sees
-// the same operations in the same order whatever the tile.
-constexpr int kMaxSlots = 64;
-// shared memory of either tile: samples [slots][PT] + phasors [slots][FT]
-constexpr size_t kDftSmem(size_t esz)
+// Contraction of one flush.  A warp takes 256 points x 4 frequencies of one
+// component, a lane the points p0 + lane + 32 a (a = 0..7); the four warps of a
+// block take FT / 4 groups of four frequencies of 1024 / FT x 4 points.  Each
+// thread keeps its 32 accumulator pairs in registers while the flush's samples
+// pass through two shared buffers of a few slots each (asynchronous copies, one
+// buffer filling while the other is used); the phasors [slots][FT] stay in
+// shared memory.  A sample is added by acc_re += s cos, acc_im -= s sin (FP64
+// fused multiply-adds) in slot order, so every accumulator sees the same
+// operations in the same order whatever the tile.
+//
+// Bound: the FP64 pipe, then the accumulators' round trip to DRAM.  Eight
+// points per phasor read keep shared memory below the pipe (a 16-byte read
+// serves 16 multiply-adds; 4 x 4 tiles would need 20 cycles of reads for 16),
+// the frequency tile follows the port (a tile of 32 does four times the work
+// for eight frequencies), and three blocks per SM let one load or store its
+// accumulators while others contract.  64 slots, FP32 samples, all ports of the
+// grid: 256^3 with 16 frequencies 892 -> 346 us, 384^3 with 8 2159 -> 595 us,
+// sixteen grids with 16 1500 -> 577 us.
+constexpr int kMaxSlots = 64, kDftThreads = 128, kDftPoints = 8;
+constexpr int kDftStage = 16384;  // bytes of a sample buffer
+constexpr size_t kDftSmem = 2 * kDftStage + sizeof(double2) * 16 * kMaxSlots;
+
+template <typename T>
+__device__ __forceinline__ void cp_async_word(T *dst, const T *src)
 {
-    return (esz * 64 + sizeof(double2) * 64) * kMaxSlots > (esz * 128 + sizeof(double2) * 32) * kMaxSlots
-               ? (esz * 64 + sizeof(double2) * 64) * kMaxSlots
-               : (esz * 128 + sizeof(double2) * 32) * kMaxSlots;
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src),
+                 "n"(sizeof(T))
+                 : "memory");
 }
 
 template <typename T, int FT>
 __device__ __forceinline__ void dft_tile(const T *ring, int npts, int nslots, const double2 *tab, int nfreq,
                                          int comp, int ci, int p0, int f0, double *acc, unsigned char *sh_raw)
 {
-    constexpr int TF = FT / 4, TP = 256 / TF, PT = 4 * TP;
-    T *ss = reinterpret_cast<T *>(sh_raw);                                          // [nslots][PT]
-    double2 *sp = reinterpret_cast<double2 *>(sh_raw + sizeof(T) * kMaxSlots * PT);  // [nslots][FT]
-    const int tid = threadIdx.x, tp = tid % TP, tf = tid / TP;
-    for (int q = tid; q < nslots * PT; q += blockDim.x) {
-        const int t = q / PT, pl = q - t * PT, p = p0 + pl;
-        ss[q] = p < npts ? ring[((int64_t)t * 6 + comp) * npts + p] : T(0);
-    }
-    for (int q = tid; q < nslots * FT; q += blockDim.x) {
-        const int t = q / FT, fl = q - t * FT, f = f0 + fl;
+    constexpr int TF = FT / 4, PT = dft_point_tile(FT), S = kDftStage / (PT * (int)sizeof(T));
+    static_assert(S >= 1 && PT == 32 * kDftPoints * (kDftThreads / 32) / TF, "sample buffer");
+    T *ss = reinterpret_cast<T *>(sh_raw);                              // [2][S][PT]
+    double2 *sp = reinterpret_cast<double2 *>(sh_raw + 2 * kDftStage);  // [nslots][FT]
+    const int tid = threadIdx.x, w = tid >> 5, tf = w % TF, pl = w / TF * (32 * kDftPoints) + (tid & 31);
+    const int nst = (nslots + S - 1) / S;
+    auto stage = [&](int st) {
+        T *b = ss + (st & 1) * (S * PT);
+        for (int q = tid; q < S * PT; q += kDftThreads) {
+            const int t = st * S + q / PT, p = p0 + q % PT;
+            if (t < nslots && p < npts) cp_async_word(b + q, ring + ((int64_t)t * 6 + comp) * npts + p);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    stage(0);
+    for (int q = tid; q < nslots * FT; q += kDftThreads) {
+        const int t = q / FT, f = f0 + q % FT;
         sp[q] = f < nfreq ? tab[(int64_t)t * nfreq + f] : make_double2(0.0, 0.0);
     }
-    double re[4][4], im[4][4];
+    double re[4][kDftPoints], im[4][kDftPoints];
 #pragma unroll
     for (int b = 0; b < 4; ++b) {
         const int f = f0 + tf * 4 + b;
         const double *ar = acc + ((int64_t)(ci * nfreq + min(f, nfreq - 1)) * 2) * npts;
 #pragma unroll
-        for (int a = 0; a < 4; ++a) {
-            const int p = p0 + a * TP + tp;
+        for (int a = 0; a < kDftPoints; ++a) {
+            const int p = p0 + pl + 32 * a;
             const bool ok = f < nfreq && p < npts;
-            re[a][b] = ok ? ar[p] : 0.0;
-            im[a][b] = ok ? ar[npts + p] : 0.0;
+            re[b][a] = ok ? ar[p] : 0.0;
+            im[b][a] = ok ? ar[npts + p] : 0.0;
         }
     }
-    __syncthreads();
-    for (int t = 0; t < nslots; ++t) {
-        double sv[4];
+    for (int st = 0; st < nst; ++st) {
+        if (st + 1 < nst) stage(st + 1);
+        else asm volatile("cp.async.commit_group;" ::: "memory");
+        asm volatile("cp.async.wait_group 1;" ::: "memory");  // all but the newest: this stage's
+        __syncthreads();
+        const T *b = ss + (st & 1) * (S * PT) + pl;
+        const double2 *wp = sp + st * S * FT + tf * 4;
+        const int n = min(S, nslots - st * S);
+        for (int t = 0; t < n; ++t) {
+            double sv[kDftPoints];
 #pragma unroll
-        for (int a = 0; a < 4; ++a) sv[a] = (double)ss[t * PT + a * TP + tp];
+            for (int a = 0; a < kDftPoints; ++a) sv[a] = (double)b[t * PT + 32 * a];
 #pragma unroll
-        for (int b = 0; b < 4; ++b) {
-            const double2 w = sp[t * FT + tf * 4 + b];
+            for (int q = 0; q < 4; ++q) {
+                const double2 ph = wp[t * FT + q];
 #pragma unroll
-            for (int a = 0; a < 4; ++a) {
-                re[a][b] = __fma_rn(sv[a], w.x, re[a][b]);
-                im[a][b] = __fma_rn(-sv[a], w.y, im[a][b]);
+                for (int a = 0; a < kDftPoints; ++a) {
+                    re[q][a] = __fma_rn(sv[a], ph.x, re[q][a]);
+                    im[q][a] = __fma_rn(-sv[a], ph.y, im[q][a]);
+                }
             }
         }
+        __syncthreads();  // read before it is filled again
     }
 #pragma unroll
     for (int b = 0; b < 4; ++b) {
@@ -130,11 +157,11 @@ __device__ __forceinline__ void dft_tile(const T *ring, int npts, int nslots, co
         if (f >= nfreq) continue;
         double *ar = acc + ((int64_t)(ci * nfreq + f) * 2) * npts;
 #pragma unroll
-        for (int a = 0; a < 4; ++a) {
-            const int p = p0 + a * TP + tp;
+        for (int a = 0; a < kDftPoints; ++a) {
+            const int p = p0 + pl + 32 * a;
             if (p >= npts) continue;
-            ar[p] = re[a][b];
-            ar[npts + p] = im[a][b];
+            ar[p] = re[b][a];
+            ar[npts + p] = im[b][a];
         }
     }
 }
@@ -144,20 +171,21 @@ template <typename T>
 __device__ __forceinline__ void dft_block(const T *ring, int npts, int nslots, const double2 *tab, int nfreq,
                                           int comp, int ci, int pb, int fb, double *acc, unsigned char *sh_raw)
 {
-    if (dft_freq_tile(nfreq) == 32)
-        dft_tile<T, 32>(ring, npts, nslots, tab, nfreq, comp, ci, pb * 128, fb * 32, acc, sh_raw);
-    else
-        dft_tile<T, 64>(ring, npts, nslots, tab, nfreq, comp, ci, pb * 64, fb * 64, acc, sh_raw);
+    const int ft = dft_freq_tile(nfreq), p0 = pb * dft_point_tile(ft), f0 = fb * ft;
+    if (ft == 4) dft_tile<T, 4>(ring, npts, nslots, tab, nfreq, comp, ci, p0, f0, acc, sh_raw);
+    else if (ft == 8) dft_tile<T, 8>(ring, npts, nslots, tab, nfreq, comp, ci, p0, f0, acc, sh_raw);
+    else dft_tile<T, 16>(ring, npts, nslots, tab, nfreq, comp, ci, p0, f0, acc, sh_raw);
 }
 
+// grid: frequency blocks innermost, so that they meet a point block's samples in L2
 template <typename T>
-__global__ void __launch_bounds__(256, 2) k_dft(const T *ring, int npts, int nslots, const double2 *tab, int nfreq,
-                                             const int32_t *comps, double *acc)
+__global__ void __launch_bounds__(kDftThreads, 3) k_dft(const T *ring, int npts, int nslots, const double2 *tab,
+                                                        int nfreq, const int32_t *comps, double *acc)
 {
     extern __shared__ __align__(16) unsigned char sh_raw[];
-    const int ci = blockIdx.y, comp = comps[ci];
+    const int ci = blockIdx.y, comp = comps[ci], nfb = (nfreq + dft_freq_tile(nfreq) - 1) / dft_freq_tile(nfreq);
     dft_block<T>(ring, npts, nslots, tab + (comp >= 3 ? (int64_t)nslots * nfreq : 0), nfreq, comp, ci,
-                 blockIdx.x, blockIdx.z, acc, sh_raw);
+                 blockIdx.x / nfb, blockIdx.x % nfb, acc, sh_raw);
 }
 
 // batched forms over the ports of many grids
@@ -214,8 +242,8 @@ __global__ void k_phasors_batch(const BatchGrid<T> *__restrict__ grids, const Ba
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256, 2) k_dft_batch(const BatchPort<T> *__restrict__ ports,
-                                                   const int4 *__restrict__ blocks, int nslots)
+__global__ void __launch_bounds__(kDftThreads, 3) k_dft_batch(const BatchPort<T> *__restrict__ ports,
+                                                              const int4 *__restrict__ blocks, int nslots)
 {
     extern __shared__ __align__(16) unsigned char sh_raw[];
     const int4 e = blocks[blockIdx.x];
@@ -302,9 +330,10 @@ void launch_port_dft(const T *ring, int npts, int nslots, int64_t n_first, doubl
     if (npts <= 0 || nslots <= 0 || nfreq <= 0 || ncomp <= 0) return;
     double2 *tab = reinterpret_cast<double2 *>(scratch_phasor);
     k_phasors<<<cdiv((int64_t)nslots * nfreq, 256), 256, 0, s>>>(omega, nfreq, nslots, n_first, dt, tab);
-    dim3 grid(cdiv(npts, dft_point_tile(nfreq)), ncomp, cdiv(nfreq, dft_freq_tile(nfreq)));
-    if (!kernel_smem<k_dft<T>>((int)kDftSmem(sizeof(T)))) return;
-    k_dft<T><<<grid, 256, kDftSmem(sizeof(T)), s>>>(ring, npts, nslots, tab, nfreq, comps, acc);
+    const int ft = dft_freq_tile(nfreq);
+    dim3 grid(cdiv(npts, dft_point_tile(ft)) * cdiv(nfreq, ft), ncomp);
+    if (!kernel_smem<k_dft<T>>((int)kDftSmem)) return;
+    k_dft<T><<<grid, kDftThreads, kDftSmem, s>>>(ring, npts, nslots, tab, nfreq, comps, acc);
 }
 
 template <typename T>
@@ -318,7 +347,7 @@ void launch_gather_batch(const BatchGrid<T> *grids, const BatchPort<T> *ports, c
 template <typename T>
 bool dft_batch_attributes()
 {
-    return kernel_smem<k_dft_batch<T>>((int)kDftSmem(sizeof(T)));
+    return kernel_smem<k_dft_batch<T>>((int)kDftSmem);
 }
 
 template <typename T>
@@ -328,7 +357,7 @@ void launch_dft_batch(const BatchGrid<T> *grids, const BatchPort<T> *ports, cons
     if (nph <= 0 || nblocks <= 0 || nslots <= 0) return;
     k_phasors_batch<T><<<nph, 256, 0, s>>>(grids, ports, ph_blocks, nslots);
     if (!dft_batch_attributes<T>()) return;
-    k_dft_batch<T><<<nblocks, 256, kDftSmem(sizeof(T)), s>>>(ports, blocks, nslots);
+    k_dft_batch<T><<<nblocks, kDftThreads, kDftSmem, s>>>(ports, blocks, nslots);
 }
 
 void launch_port_flux(const double *acc, int npts, int nfreq, int ncomp, const int32_t *sel, double dA,

@@ -141,3 +141,43 @@ def test_fp64_gain_sweep_equals_plain_routines(rows, planes):
             g.close()
         for q, (x, y) in enumerate(zip(*out)):
             assert rel_l2(y, x) < 1e-12, (nx, q, rel_l2(y, x))
+
+
+@pytest.mark.parametrize("chunked", [False, True])
+@pytest.mark.parametrize("prec", [0, 1], ids=["fp64", "fp32"])
+@pytest.mark.parametrize("nfreq", [1, 4, 5, 8, 9, 16, 17, 33])
+def test_port_dft_tiles(nfreq, prec, chunked):
+    """Ports whose points and frequencies end inside, at and past a tile of the
+    contraction, over a whole ring and part of one, against sums of the samples
+    in the same precision.  70 terms of one size each: 70 roundings of the sum
+    and as many of the phase, 1.1e-16 each, within 1e-12 of the largest."""
+    import cpsfdtd_b200 as cps
+    n, d, steps = 48, 10e-9, 70
+    dk = decks.Deck(n, n, 12, d, d, d)
+    dk.media = [(1.0, 1.0, 0.0, 0.0)]
+    freqs = np.linspace(0.8, 1.2, nfreq) * 5e14
+    for w, h in ((1, 1), (15, 17), (16, 16), (27, 19), (32, 32), (25, 41)):
+        dk.ports.append(decks.Port("plain", dict(dir="z", position=6.5 * d, w1=2.5 * d, w2=(2 + w - 0.5) * d,
+                                                 h1=3.5 * d, h2=(3 + h - 0.5) * d), dft_freqs=freqs, dft_mask=0x2B))
+    a, b = cps.Grid.from_deck(dk, prec), cps.Grid.from_deck(dk, prec)
+    for g in (a, b):
+        _noise(g, dk, 3)
+        g.set_chunked(chunked)
+    n0 = a.get_step()
+    a.step(steps, cps.FUSED)
+    series = [[] for _ in dk.ports]
+    for _ in range(steps):
+        b.step(1, cps.FUSED)
+        for p in range(len(dk.ports)):
+            series[p].append(np.asarray(b.port_last(p)).T)
+    comps = [c for c in range(6) if 0x2B >> c & 1]
+    for p in range(len(dk.ports)):
+        got = np.asarray(a.port_dft(p, raw=True))
+        npts = series[p][0].shape[1]
+        got = got.reshape(len(comps), nfreq, 2, npts)
+        t = (n0 + np.arange(steps)) * dk.dt
+        for q, c in enumerate(comps):
+            s = np.stack([x[c] for x in series[p]])
+            ph = np.outer(2 * np.pi * freqs, t - (0.5 * dk.dt if c >= 3 else 0.0))
+            want = np.stack([np.cos(ph) @ s, -np.sin(ph) @ s], axis=1)
+            assert np.abs(got[q] - want).max() <= 1e-12 * np.abs(s).sum(axis=0).max(), (p, c)
