@@ -259,16 +259,7 @@ cps_status rebuild_T(cps_batch *b)
         B.p = pml_view<T>(g);
         B.D = dl_view<T>(g);
         B.G = gain_view<T>(g);
-        if (g->tfsf_on) {
-            for (int side = 0; side < 2; ++side) {
-                B.tg[side] = g->d_tg[side];
-                B.ct[side] = g->d_ct[side];
-                B.ntg[side] = g->ntg[side];
-            }
-            B.inc[0] = (const T *)g->d_hinc;
-            B.inc[1] = (const T *)g->d_einc;
-            B.Nt = g->tp.Nt;
-        }
+        for (int side = 0; side < 2; ++side) B.inj[side] = inj_view<T>(g, side);
         B.nsrc = (int)g->src.size();
         B.src_idx = g->d_src_idx; B.src_comp = g->d_src_comp; B.src_off = g->d_src_off;
         B.src_len = g->d_src_len; B.src_wave = g->d_src_wave;
@@ -309,8 +300,8 @@ cps_status rebuild_T(cps_batch *b)
                 dl.push_back(make_int4((int)gi, (int)c0, (int)std::min<int64_t>(c0 + 128, B.D.ncell), 0));
         }
         for (int side = 0; side < 2; ++side)
-            for (int t0 = 0; t0 < B.ntg[side]; t0 += kInjPerBlock)
-                inj[side].push_back(make_int4((int)gi, t0, std::min(t0 + kInjPerBlock, B.ntg[side]), 0));
+            for (int t0 = 0; t0 < B.inj[side].n; t0 += kInjPerBlock)
+                inj[side].push_back(make_int4((int)gi, t0, std::min(t0 + kInjPerBlock, B.inj[side].n), 0));
         for (int q = 0; q < B.nsrc; ++q) src.push_back(make_int2((int)gi, q));
         for (PortState &P : g->ports) {
             BatchPort<T> bp;
@@ -406,6 +397,34 @@ FusedShape member_shape(const cps_batch *b, const cps_grid *g)
     return sh;
 }
 
+// Port samples of step s of a one-grid chunk whose last step is `last`: what
+// k_gather_batch takes, with the pointers as kernel parameters.  Returns the
+// launch count.
+template <typename T>
+int gather_one(const cps_grid *g, int s, int last, cudaStream_t st)
+{
+    int n = 0;
+    GatherBatch B;
+    memset(&B, 0, sizeof(B));
+    auto flush = [&] {
+        if (B.max_npts > 0) launch_port_gather<T>(field_view<T>(g), B, false, st), ++n;
+        memset(&B, 0, sizeof(B));
+    };
+    for (const PortState &P : g->ports) {
+        if (P.npts <= 0 || (s != last && P.slots == 1)) continue;
+        GatherDesc &D = B.p[B.n++];
+        D.idx = P.d_idx;
+        D.slot = (T *)P.d_ring + (int64_t)(P.slots == 1 ? 0 : s) * 6 * P.npts;
+        D.npts = P.npts;
+        if (s == last) D.comps = 0x3F;
+        else for (int c = 0; c < P.ncomp; ++c) D.comps |= 1 << P.comps[c];
+        B.max_npts = std::max(B.max_npts, P.npts);
+        if (B.n == kMaxGather) flush();
+    }
+    flush();
+    return n;
+}
+
 // Enqueue one chunk of S steps on the batch stream; returns the launch count.
 template <typename T>
 int64_t enqueue_chunk(cps_batch *b, int S)
@@ -415,13 +434,20 @@ int64_t enqueue_chunk(cps_batch *b, int S)
     cudaStream_t st = b->stream;
     int64_t n = 0;
     for (int s = 0; s < S; ++s) {
+        // one grid: its pointers as kernel parameters, not through the tables
+        auto inject = [&](int side) {
+            if (b->grids.size() == 1)
+                launch_inject_all<T>(field_view<T>(b->grids[0]), inj_view<T>(b->grids[0], side), &G[0].n0, s, false, st);
+            else
+                launch_inject_batch<T>(G, b->d_inj[side], b->ninj[side], side, s, st);
+        };
         launch_h_batch<T>(G, b->d_tiles[kHInt], b->ntiles[kHInt], b->nblocks[kHInt], b->by, false, b->d_err, st);
         launch_h_batch<T>(G, b->d_tiles[kHPml], b->ntiles[kHPml], b->nblocks[kHPml], b->by, true, b->d_err, st);
         per_member(b, [&](int gi, cudaStream_t ms) {
             const cps_grid *g = b->grids[gi];
             n += launch_h_tma<T>(g->tma, field_view<T>(g), pml_view<T>(g), member_shape(b, g), b->d_err, ms);
         });
-        launch_inject_batch<T>(G, b->d_inj[1], b->ninj[1], 1, s, st);
+        inject(1);
         for (int c = 0; c < 8; ++c)
             launch_e_batch<T>(G, b->d_tiles[kE0 + c], b->ntiles[kE0 + c], b->nblocks[kE0 + c], b->by, c, b->d_err, st);
         launch_dl_batch<T>(G, b->d_dl, b->ndl, st);
@@ -430,13 +456,14 @@ int64_t enqueue_chunk(cps_batch *b, int S)
             n += launch_e_tma<T>(g->tma, field_view<T>(g), pml_view<T>(g), dl_view<T>(g), gain_view<T>(g),
                             member_shape(b, g), b->d_err, ms, &g->lane);
         });
-        launch_inject_batch<T>(G, b->d_inj[0], b->ninj[0], 0, s, st);
+        inject(0);
         launch_sources_batch<T>(G, b->d_src, b->nsrc, s, st);
         // without a port DFT only the chunk's last sample is kept
         const bool sample = b->ndft > 0 || s == S - 1;
-        if (sample) launch_gather_batch<T>(G, P, b->d_gather, b->ngather, s, S - 1, st);
+        if (sample && b->grids.size() == 1) n += gather_one<T>(b->grids[0], s, S - 1, st);
+        else if (sample) launch_gather_batch<T>(G, P, b->d_gather, b->ngather, s, S - 1, st), n += b->ngather > 0;
         for (int c = 0; c < kNumSweep; ++c) n += b->ntiles[c] > 0;
-        n += (b->ndl > 0) + (b->ninj[0] > 0) + (b->ninj[1] > 0) + (b->nsrc > 0) + (sample && b->ngather > 0);
+        n += (b->ndl > 0) + (b->ninj[0] > 0) + (b->ninj[1] > 0) + (b->nsrc > 0);
     }
     launch_dft_batch<T>(G, P, b->d_phasor, b->nphasor, b->d_dft, b->ndft, S, st);
     n += b->ndft > 0 ? 2 : 0;

@@ -22,11 +22,7 @@ struct alignas(64) BatchGrid {
     PmlView<T> p;
     DlView<T> D;
     GainView<T> G;
-    const InjTarget *tg[2];   // TF/SF targets: [0] E side, [1] H side
-    const InjContrib *ct[2];
-    const T *inc[2];          // incident tables: [0] Hinc (E side), [1] Einc (H side)
-    int ntg[2];
-    int Nt;
+    InjView<T> inj[2];        // TF/SF targets: [0] E side, [1] H side
     int nsrc;
     const int64_t *src_idx;
     const int32_t *src_comp, *src_off, *src_len;

@@ -296,8 +296,11 @@ void op_inject(cps_grid *g, int isH, double n, uint32_t mask)
 {
     if (!g->tfsf_on || g->ntg[isH] == 0) return;
     const FieldView<T> f = field_view<T>(g);
-    launch_inject<T>(f, g->d_tg[isH], g->ntg[isH], g->d_ct[isH], (const T *)(isH ? g->d_einc : g->d_hinc),
-                     g->tp.Nt, n, mask, g->stream);
+    if ((mask & CPS_FACE_ALL) == CPS_FACE_ALL)
+        launch_inject_all<T>(f, inj_view<T>(g, isH), nullptr, (int64_t)n, true, g->stream);
+    else
+        launch_inject<T>(f, g->d_tg[isH], g->ntg[isH], g->d_ct[isH], (const T *)(isH ? g->d_einc : g->d_hinc),
+                         g->tp.Nt, n, mask, g->stream);
     g->launches++;
 }
 
@@ -329,12 +332,13 @@ cps_status op_ports(cps_grid *g, PortState *const *ports, int nports, int64_t n,
             D.idx = P.d_idx;
             D.slot = (T *)P.d_ring + (int64_t)P.fill * 6 * P.npts;
             D.npts = P.npts;
+            D.comps = 0x3F;
             B.max_npts = std::max(B.max_npts, P.npts);
             P.last_slot = P.fill;
             P.fill++;
             if (P.nfreq == 0) P.fill = 0;  // no DFT: the ring holds the last sample only
         }
-        launch_port_gather<T>(field_view<T>(g), B, g->stream);
+        launch_port_gather<T>(field_view<T>(g), B, true, g->stream);
         g->launches++;
     }
     return CPS_OK;
@@ -1392,6 +1396,9 @@ extern "C" cps_status cps_tfsf_init(cps_grid *g, const cps_tfsf_params *p)
         if ((s = dalloc(g, (void **)&g->d_ct[side], ct.size() * sizeof(InjContrib)))) return s;
         if ((s = upload_raw(g, g->d_tg[side], tg.data(), tg.size() * sizeof(InjTarget)))) return s;
         if ((s = upload_raw(g, g->d_ct[side], ct.data(), ct.size() * sizeof(InjContrib)))) return s;
+        if ((s = dalloc(g, &g->d_inj[side], inj_pack_bytes((int)tg.size(), g->esz)))) return s;
+        if (g->fp32) launch_inject_pack<float>(g->d_inj[side], g->d_tg[side], g->ntg[side], g->d_ct[side], g->stream);
+        else launch_inject_pack<double>(g->d_inj[side], g->d_tg[side], g->ntg[side], g->d_ct[side], g->stream);
     }
     // incident tables, TF_SF.cpp:898-955
     const int Nt = p->Nt;

@@ -54,6 +54,11 @@ struct Dims {
     }
 };
 
+template <typename T>
+struct alignas(2 * sizeof(T)) Pair {
+    T a, b;
+};
+
 // --- Drude-Lorentz coefficients (host FP64, converted to T for the device)
 template <typename T>
 struct DlCoef {
@@ -265,6 +270,35 @@ void launch_three_init(const ThreeView &t, double N_0, cudaStream_t s);
 template <typename T>
 void launch_inject(const FieldView<T> &f, const InjTarget *tg, int ntarget, const InjContrib *ct,
                    const T *table, int Nt, double n, uint32_t face_mask, cudaStream_t s);
+// One side's targets as the step reads them: word = index | component << 48 |
+// (more than one contribution) << 51, and the first contribution beside it, so
+// that all but the box's edges take one round of loads before the incident
+// table and the field.  Further contributions come from the CSR lists.
+template <typename T>
+struct InjView {
+    const uint64_t *word;
+    const double *delay;
+    const Pair<T> *cp;  // (coef, profile)
+    const InjTarget *tg;
+    const InjContrib *ct;
+    const T *table;
+    int n, Nt;
+};
+inline size_t inj_pack_bytes(int n, size_t esz) { return (size_t)n * (16 + 2 * esz); }
+template <typename T>
+inline void inj_pack_view(InjView<T> &v, void *pack, int n)
+{
+    v.n = n;
+    v.word = (const uint64_t *)pack;
+    v.delay = (const double *)(v.word + n);
+    v.cp = (const Pair<T> *)(v.delay + n);
+}
+template <typename T>
+void launch_inject_pack(void *pack, const InjTarget *tg, int ntarget, const InjContrib *ct, cudaStream_t s);
+// every face at step (n0 ? *n0 : 0) + n; early: see launch_pdl
+template <typename T>
+void launch_inject_all(const FieldView<T> &f, const InjView<T> &v, const int64_t *n0, int64_t n, bool early,
+                       cudaStream_t s);
 template <typename T>
 void launch_sources(const FieldView<T> &f, int nsrc, const int64_t *idx, const int32_t *comp,
                     const double *waves, const int32_t *wave_off, const int32_t *wave_len, int n,
@@ -341,7 +375,7 @@ struct GatherDesc {
     const int64_t *idx;
     void *slot;  // ring slot [6][npts] of T
     int npts;
-    int pad;
+    int comps;   // components to sample, a bit each
 };
 struct GatherBatch {
     GatherDesc p[kMaxGather];
@@ -349,7 +383,7 @@ struct GatherBatch {
     int max_npts;
 };
 template <typename T>
-void launch_port_gather(const FieldView<T> &f, const GatherBatch &b, cudaStream_t s);
+void launch_port_gather(const FieldView<T> &f, const GatherBatch &b, bool early, cudaStream_t s);
 template <typename T>
 void launch_port_dft(const T *ring, int npts, int nslots, int64_t n_first, double dt,
                      const double *omega, int nfreq, const int32_t *comps, int ncomp,

@@ -135,6 +135,7 @@ struct cps_grid {
     void *d_einc = nullptr, *d_hinc = nullptr;
     InjTarget *d_tg[2] = {nullptr, nullptr};   // 0: E targets, 1: H targets
     InjContrib *d_ct[2] = {nullptr, nullptr};
+    void *d_inj[2] = {nullptr, nullptr};       // the targets as the step reads them (InjView)
     int ntg[2] = {0, 0};
     // sources
     std::vector<Src> src;
@@ -241,6 +242,20 @@ inline FieldView<T> field_view(const cps_grid *g)
     f.aE = m; f.bE = m + 256; f.aH = m + 512; f.bH = m + 768;
     f.s = stretch_view<T>(g);
     return f;
+}
+
+template <typename T>
+inline InjView<T> inj_view(const cps_grid *g, int isH)
+{
+    InjView<T> v;
+    memset(&v, 0, sizeof(v));
+    if (!g->tfsf_on) return v;
+    inj_pack_view(v, g->d_inj[isH], g->ntg[isH]);
+    v.tg = g->d_tg[isH];
+    v.ct = g->d_ct[isH];
+    v.table = (const T *)(isH ? g->d_einc : g->d_hinc);
+    v.Nt = g->tp.Nt;
+    return v;
 }
 
 // the second field buffer set of the one-pass step (written by the next step)

@@ -337,13 +337,66 @@ __global__ void k_inject(FieldView<T> f, const InjTarget *tg, int ntarget, const
     inject_target<T>(f, tg[t], ct, table, Nt, n, face_mask);
 }
 
-// batched forms: the step number is the grid's chunk start plus step_off.
-// A block entry covers kInjPerBlock targets; each thread takes two of them,
-// kInjThreads apart, and requests both targets' records, field values and
-// first contributions before using any (the kernel is bound by the latency
-// of these dependent loads).  Each target's contributions are added in its
-// own order, as in inject_target; the two targets are distinct (cell,
-// component) pairs, so their updates are independent.
+template <typename T>
+__global__ void k_inject_pack(uint64_t *word, double *delay, Pair<T> *cp, const InjTarget *tg, int ntarget,
+                              const InjContrib *ct)
+{
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= ntarget) return;
+    const InjTarget q = tg[t];
+    const InjContrib a = ct[q.start];  // every target has at least one contribution
+    word[t] = (uint64_t)q.idx | (uint64_t)q.comp << 48 | (q.count > 1 ? 1ull << 51 : 0ull);
+    delay[t] = a.delay;
+    cp[t] = Pair<T>{(T)a.coef, (T)a.profile};
+}
+
+// Every face of one side.  A few megabytes move, so what bounds this is the
+// chain of dependent loads; each thread takes two targets kInjThreads apart and
+// asks for both at every link.  With the first contribution beside the target
+// and the grid's pointers as kernel parameters the chain is record, then table
+// and field: 256^3 (580 k targets a side), 16.3 -> 12.4 us; through the CSR
+// lists and a descriptor it was block, grid, target, contribution, table.
+// Each target's contributions are added in its own order, as in inject_target;
+// the two targets are distinct (cell, component) pairs.
+template <typename T>
+__device__ __forceinline__ void inject_two(const FieldView<T> &f, const InjView<T> &V, int t0, int end, double n)
+{
+    if (t0 >= end) return;
+    const int t1 = t0 + kInjThreads;
+    const bool two = t1 < end;
+    const int u1 = two ? t1 : t0;
+    const uint64_t w0 = V.word[t0], w1 = V.word[u1];
+    const double d0 = V.delay[t0], d1 = V.delay[u1];
+    const Pair<T> c0 = V.cp[t0], c1 = V.cp[u1];
+    const uint64_t mask = (1ull << 48) - 1;
+    T *F0 = field_comp(f, (int)(w0 >> 48 & 7)) + (w0 & mask);
+    T *F1 = field_comp(f, (int)(w1 >> 48 & 7)) + (w1 & mask);
+    T v0 = *F0, v1 = *F1;
+    v0 = v0 + c0.a * (T)inc_lookup<T>(V.table, V.Nt, n - d0) * c0.b;
+    v1 = v1 + c1.a * (T)inc_lookup<T>(V.table, V.Nt, n - d1) * c1.b;
+    auto rest = [&](int t, T v) {
+        const InjTarget q = V.tg[t];
+        for (int c = q.start + 1; c < q.start + q.count; ++c) v = inject_add(v, V.ct[c], V.table, V.Nt, n);
+        return v;
+    };
+    if (w0 >> 51) v0 = rest(t0, v0);
+    *F0 = v0;
+    if (!two) return;
+    if (w1 >> 51) v1 = rest(t1, v1);
+    *F1 = v1;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kInjThreads) k_inject_all(FieldView<T> f, InjView<T> V, const int64_t *n0, int64_t n)
+{
+    pdl_go();
+    pdl_wait();
+    inject_two<T>(f, V, blockIdx.x * kInjPerBlock + (int)threadIdx.x, min((int)(blockIdx.x + 1) * kInjPerBlock, V.n),
+                  (double)((n0 ? *n0 : 0) + n));
+}
+
+// batched form: the step number is the grid's chunk start plus step_off; a
+// block entry covers up to kInjPerBlock targets
 template <typename T>
 __global__ void __launch_bounds__(kInjThreads) k_inject_batch(const BatchGrid<T> *__restrict__ grids,
                                                               const int4 *__restrict__ blocks, int side,
@@ -352,30 +405,8 @@ __global__ void __launch_bounds__(kInjThreads) k_inject_batch(const BatchGrid<T>
     pdl_go();
     pdl_wait();
     const int4 e = blocks[blockIdx.x];
-    const int t0 = e.y + (int)threadIdx.x, t1 = t0 + kInjThreads;
-    if (t0 >= e.z) return;
-    const bool two = t1 < e.z;
     const BatchGrid<T> &B = grids[e.x];
-    const InjTarget *tg = B.tg[side];
-    const InjContrib *ct = B.ct[side];
-    const T *table = B.inc[side];
-    const int Nt = B.Nt;
-    const double n = (double)(B.n0 + step_off);
-    const InjTarget q0 = tg[t0];
-    const InjTarget q1 = two ? tg[t1] : q0;
-    T *F0 = field_comp(B.f, q0.comp) + q0.idx;
-    T *F1 = field_comp(B.f, q1.comp) + q1.idx;
-    T v0 = *F0;
-    T v1 = two ? *F1 : T(0);
-    const InjContrib a0 = ct[q0.start];  // every target has at least one contribution
-    const InjContrib a1 = ct[q1.start];
-    v0 = inject_add(v0, a0, table, Nt, n);
-    for (int c = q0.start + 1; c < q0.start + q0.count; ++c) v0 = inject_add(v0, ct[c], table, Nt, n);
-    *F0 = v0;
-    if (!two) return;
-    v1 = inject_add(v1, a1, table, Nt, n);
-    for (int c = q1.start + 1; c < q1.start + q1.count; ++c) v1 = inject_add(v1, ct[c], table, Nt, n);
-    *F1 = v1;
+    inject_two<T>(B.f, B.inj[side], e.y + (int)threadIdx.x, e.z, (double)(B.n0 + step_off));
 }
 
 template <typename T>
@@ -513,6 +544,24 @@ void launch_inject(const FieldView<T> &f, const InjTarget *tg, int ntarget, cons
 }
 
 template <typename T>
+void launch_inject_pack(void *pack, const InjTarget *tg, int ntarget, const InjContrib *ct, cudaStream_t s)
+{
+    if (ntarget <= 0) return;
+    InjView<T> v;
+    inj_pack_view(v, pack, ntarget);
+    k_inject_pack<T><<<cdiv(ntarget, 256), 256, 0, s>>>((uint64_t *)v.word, (double *)v.delay, (Pair<T> *)v.cp, tg,
+                                                        ntarget, ct);
+}
+
+template <typename T>
+void launch_inject_all(const FieldView<T> &f, const InjView<T> &v, const int64_t *n0, int64_t n, bool early,
+                       cudaStream_t s)
+{
+    if (v.n <= 0) return;
+    launch_pdl(early, k_inject_all<T>, cdiv(v.n, kInjPerBlock), kInjThreads, 0, s, f, v, n0, n);
+}
+
+template <typename T>
 void launch_sources(const FieldView<T> &f, int nsrc, const int64_t *idx, const int32_t *comp,
                     const double *waves, const int32_t *wave_off, const int32_t *wave_len, int n,
                     cudaStream_t s)
@@ -543,6 +592,9 @@ void launch_sources_batch(const BatchGrid<T> *grids, const int2 *ents, int n, in
     template void launch_e_pml<T>(const FieldView<T> &, const PmlView<T> &, cudaStream_t);              \
     template void launch_dl<T>(const FieldView<T> &, const DlView<T> &, cudaStream_t);                  \
     template void launch_gain<T>(const FieldView<T> &, const GainView<T> &, int, cudaStream_t);         \
+    template void launch_inject_pack<T>(void *, const InjTarget *, int, const InjContrib *, cudaStream_t); \
+    template void launch_inject_all<T>(const FieldView<T> &, const InjView<T> &, const int64_t *, int64_t, bool, \
+                                       cudaStream_t);                                                    \
     template void launch_inject<T>(const FieldView<T> &, const InjTarget *, int, const InjContrib *,    \
                                    const T *, int, double, uint32_t, cudaStream_t);                     \
     template void launch_sources<T>(const FieldView<T> &, int, const int64_t *, const int32_t *,        \
