@@ -747,9 +747,12 @@ cps_status step_T(cps_grid *g, int nsteps, int path)
             op_sources<T>(g, (int)n);
         }
         if (!g->ports.empty()) {
+            // a port without a DFT keeps its last sample only: taken after the last
+            // step (96^3 FP64 plain, 46.0 -> 43.1 us a step)
             std::vector<PortState *> all;
-            for (PortState &P : g->ports) all.push_back(&P);
-            s = op_ports<T>(g, all.data(), (int)all.size(), n);
+            for (PortState &P : g->ports)
+                if (P.nfreq > 0 || it == nsteps - 1) all.push_back(&P);
+            if (!all.empty()) s = op_ports<T>(g, all.data(), (int)all.size(), n);
             if (s) return s;
         }
         g->step++;

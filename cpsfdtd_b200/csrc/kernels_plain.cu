@@ -14,7 +14,12 @@ namespace cps {
 
 namespace {
 
-constexpr int kBY = 8;
+// rows of a block of the bulk and CPML kernels.  A block with slab cells takes
+// several times as long as one without, so small blocks fill the SMs better:
+// 96^3 FP64 43.1, 41.0 and 45.4 us a step with 8, 4 and 2 rows.  (Requesting a
+// cell's psi words before its field words costs the registers of a third of the
+// warps: 52 us.)
+constexpr int kBY = 4;
 
 // psi index of slab-local s at (i,j,k) for axis a (x: [k][j][s], y: [k][s][i], z: [s][j][i])
 __device__ __forceinline__ int64_t psi_index(const Dims &d, int axis, int np, int s, int i, int j, int k)
