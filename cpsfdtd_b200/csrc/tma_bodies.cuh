@@ -259,11 +259,14 @@ __device__ __forceinline__ bool e_tma_body(const TmaMaps &M, const FieldView<T> 
         if (__syncthreads_or(!ok)) {
             if (tid == 0) {
                 atomicExch(err, 1);
-                drain_stages<L::NS>(full, c0, it + 1, min(it + L::NS - 1, npl - 1));
+                drain_stages<L::NS>(full, c0, it + 1, min(it + (it == 0 ? L::NS - 1 : L::NS - 2), npl - 1));
             }
             if (G64) cp_async_wait_all();
             return false;
         }
+        // every thread is past plane k - 1, so its stage takes the plane NS - 1
+        // ahead: one barrier per plane
+        if (tid == 0 && it > 0 && k - 1 + L::NS < k1) issue(it - 1 + L::NS, k - 1 + L::NS);
         const unsigned char *b = sm + s * L::STAGE_B;
         const T *hxt = (const T *)b, *hyt = (const T *)(b + L::HALO_B), *hzt = (const T *)(b + 2 * L::HALO_B);
         const T *ext = (const T *)(b + 3 * L::HALO_B), *eyt = (const T *)(b + 3 * L::HALO_B + L::OWN_B);
@@ -312,12 +315,12 @@ __device__ __forceinline__ bool e_tma_body(const TmaMaps &M, const FieldView<T> 
         qc = qn;
         qn = qnn;
         cExy = nExy; cEyx = nEyx;
-        __syncthreads();
         if constexpr (G64) {
+            __syncwarp();  // the slots are read before they are filled again
             if (PML && act && k + 1 < k1) psi_fetch_e(p, d, pc, i, j, k + 1, slot);
         }
-        if (tid == 0 && k + L::NS < k1) issue(it + L::NS, k + L::NS);
     }
+    __syncthreads();  // stages and table are free for a next tile
     ctr = c0 + (uint32_t)(k1 - k0);
     return true;
 }
@@ -391,10 +394,13 @@ __device__ __forceinline__ bool h_tma_body(const TmaMaps &M, const FieldView<T> 
             if (__syncthreads_or(!ok)) {
                 if (tid == 0) {
                     atomicExch(err, 2);
-                    drain_stages(full, c0, it + 2, min(it + kStages - 1, npl));
+                    drain_stages(full, c0, it + 2, min(it + (it == 0 ? kStages - 1 : kStages - 2), npl));
                 }
                 return false;
             }
+            // every thread is past plane k - 1, so its stage takes the plane
+            // kStages - 1 ahead: one barrier per plane
+            if (tid == 0 && it > 0 && k - 1 + kStages <= k1) issue(it - 1 + kStages, k - 1 + kStages);
             const unsigned char *b = sm + s * L::STAGE_B, *bn = sm + sn * L::STAGE_B;
             const T *ext = (const T *)b, *eyt = (const T *)(b + L::HALO_B), *ezt = (const T *)(b + 2 * L::HALO_B);
             const T *hxt = (const T *)(b + 3 * L::HALO_B), *hyt = (const T *)(b + 3 * L::HALO_B + L::OWN_B);
@@ -419,10 +425,9 @@ __device__ __forceinline__ bool h_tma_body(const TmaMaps &M, const FieldView<T> 
             }
             ex = exk; ey = eyk;
             cHxy = nHxy; cHyx = nHyx;
-            __syncthreads();
-            if (tid == 0 && k + kStages <= k1) issue(it + kStages, k + kStages);
         }
     }
+    __syncthreads();  // stages and table are free for a next tile
     ctr = c0 + (uint32_t)(k1 - k0 + 1);
     return true;
 }
