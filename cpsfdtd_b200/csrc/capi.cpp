@@ -463,7 +463,6 @@ cps_status ensure_tma(cps_grid *g)
         const cuuint32_t tb[4] = {36, (cuuint32_t)by + 1, 1, 2};
         REQUIRE(encode(&W.tail, dt, 4, other, fd, fs, tb) == CUDA_SUCCESS, CPS_E_CUDA,
                 "cuTensorMapEncodeTiled failed for a side's fields");
-        W.gain = T.gain;
         for (int f = 0; f < 6 && g->pml_on; ++f) {
             const cuuint64_t np = (cuuint64_t)g->pml.npml[f];
             const cuuint64_t row = f < 2 ? (cuuint64_t)psi_xw((int)np) : (cuuint64_t)d.px;

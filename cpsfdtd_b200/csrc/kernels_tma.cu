@@ -72,15 +72,15 @@ __global__ void __launch_bounds__(32 * BY) k_h_tma(const __grid_constant__ TmaMa
 }
 
 // blocks of one warp that fit an SM's shared memory
-template <typename T, int BY, bool GAIN>
+template <typename T, int BY>
 constexpr int warp_blocks()
 {
-    return (227 * 1024) / (warp_ring<T, BY, GAIN>() + 1024 + 640);
+    return (227 * 1024) / (warp_ring<T, BY>() + 1024 + 640);
 }
 
 // One warp per tile.  PM: 0 no CPML on the grid, 2 the body each tile needs.
 template <typename T, int BY, int PM>
-__global__ void __launch_bounds__(32, warp_blocks<T, BY, false>())
+__global__ void __launch_bounds__(32, warp_blocks<T, BY>())
     k_h_warp(const __grid_constant__ SweepMaps M, FieldView<T> f, PmlView<T> p, int kc, int nbx, int nby, int *err)
 {
     extern __shared__ __align__(128) unsigned char sm_raw[];
@@ -96,17 +96,16 @@ __global__ void __launch_bounds__(32, warp_blocks<T, BY, false>())
     if (threadIdx.x < kTab) tab[threadIdx.x] = Coef2<T>{f.aH[threadIdx.x], f.bH[threadIdx.x]};
     init_ring(full);
     pdl_wait();
-    Ring R{align_smem(sm_raw), full, warp_ring<T, BY, false>() - 128, 0u, wait_skew(err), err};
+    Ring R{align_smem(sm_raw), full, warp_ring<T, BY>() - 128, 0u, wait_skew(err), err};
     if (PM == 1 || (PM == 2 && tile_in_pml(p.np, f.d, t.bx * 32, t.by * BY, BY, k0, k1, false)))
         h_warp_tile<T, BY, 1, PM != 0>(M, f, p, kc, t, R, tab);
     else
         h_warp_tile<T, BY, kPlanes, false>(M, f, p, kc, t, R, tab);
 }
 
-template <typename T, int BY, int PM, bool DL, bool GAIN>
-__global__ void __launch_bounds__(32, warp_blocks<T, BY, GAIN>())
-    k_e_warp(const __grid_constant__ SweepMaps M, FieldView<T> f, PmlView<T> p, GainView<T> G, int kc, int nbx, int nby,
-             int *err)
+template <typename T, int BY, int PM, bool DL>
+__global__ void __launch_bounds__(32, warp_blocks<T, BY>())
+    k_e_warp(const __grid_constant__ SweepMaps M, FieldView<T> f, PmlView<T> p, int kc, int nbx, int nby, int *err)
 {
     extern __shared__ __align__(128) unsigned char sm_raw[];
     __shared__ __align__(8) uint64_t full[kMaxStages];
@@ -121,11 +120,11 @@ __global__ void __launch_bounds__(32, warp_blocks<T, BY, GAIN>())
     if (threadIdx.x < kTab) tab[threadIdx.x] = Coef2<T>{f.aE[threadIdx.x], f.bE[threadIdx.x]};
     init_ring(full);
     pdl_wait();
-    Ring R{align_smem(sm_raw), full, warp_ring<T, BY, GAIN>() - 128, 0u, wait_skew(err), err};
+    Ring R{align_smem(sm_raw), full, warp_ring<T, BY>() - 128, 0u, wait_skew(err), err};
     if (PM == 1 || (PM == 2 && tile_in_pml(p.np, f.d, t.bx * 32, t.by * BY, BY, k0, k1, true)))
-        e_warp_tile<T, BY, 1, PM != 0, DL, GAIN>(M, f, p, G, kc, t, R, tab);
+        e_warp_tile<T, BY, 1, PM != 0, DL>(M, f, p, kc, t, R, tab);
     else
-        e_warp_tile<T, BY, GAIN ? 1 : kPlanes, false, DL, GAIN>(M, f, p, G, kc, t, R, tab);
+        e_warp_tile<T, BY, kPlanes, false, DL>(M, f, p, kc, t, R, tab);
 }
 
 // The ID-2 cells the TMA E sweep leaves alone, one thread per cell of the
@@ -245,22 +244,21 @@ template <typename T, int BY, int PM>
 int h_warp_launch(const SweepMaps &M, const FieldView<T> &f, const PmlView<T> &p, int kc, int *err, cudaStream_t s)
 {
     kc = (kc + kPlanes - 1) / kPlanes * kPlanes;
-    constexpr int smem = warp_ring<T, BY, false>();
+    constexpr int smem = warp_ring<T, BY>();
     const int nbx = (int)cdiv(f.d.nx, 32), nby = (int)cdiv(f.d.ny, BY), nbz = (int)cdiv(f.d.nz, kc);
     if (!set_smem<k_h_warp<T, BY, PM>>(smem)) return 0;
     launch_pdl(true, k_h_warp<T, BY, PM>, nbx * nby * nbz, 32, smem, s, M, f, p, kc, nbx, nby, err);
     return 1;
 }
 
-template <typename T, int BY, int PM, bool DL, bool GAIN>
-int e_warp_launch(const SweepMaps &M, const FieldView<T> &f, const PmlView<T> &p, const GainView<T> &G, int kc, int *err,
-                  cudaStream_t s)
+template <typename T, int BY, int PM, bool DL>
+int e_warp_launch(const SweepMaps &M, const FieldView<T> &f, const PmlView<T> &p, int kc, int *err, cudaStream_t s)
 {
     kc = (kc + kPlanes - 1) / kPlanes * kPlanes;
-    constexpr int smem = warp_ring<T, BY, GAIN>();
+    constexpr int smem = warp_ring<T, BY>();
     const int nbx = (int)cdiv(f.d.nx, 32), nby = (int)cdiv(f.d.ny, BY), nbz = (int)cdiv(f.d.nz, kc);
-    if (!set_smem<k_e_warp<T, BY, PM, DL, GAIN>>(smem)) return 0;
-    launch_pdl(!DL, k_e_warp<T, BY, PM, DL, GAIN>, nbx * nby * nbz, 32, smem, s, M, f, p, G, kc, nbx, nby, err);
+    if (!set_smem<k_e_warp<T, BY, PM, DL>>(smem)) return 0;
+    launch_pdl(!DL, k_e_warp<T, BY, PM, DL>, nbx * nby * nbz, 32, smem, s, M, f, p, kc, nbx, nby, err);
     return 1;
 }
 
@@ -268,7 +266,7 @@ int e_warp_launch(const SweepMaps &M, const FieldView<T> &f, const PmlView<T> &p
 template <typename T, int BY>
 void attrs_by()
 {
-    constexpr int S = warp_ring<T, BY, false>(), SB = StageLayout<T, BY>::SMEM;
+    constexpr int S = warp_ring<T, BY>(), SB = StageLayout<T, BY>::SMEM;
     constexpr int SG = ELayout<T, BY, true>::SMEM;
     if constexpr (sizeof(T) == 4) {
         set_smem<k_h_warp<T, BY, 0>>(S);
@@ -277,10 +275,10 @@ void attrs_by()
         set_smem<k_h_tma<T, BY, 0>>(SB);
         set_smem<k_h_tma<T, BY, 2>>(SB);
     }
-    set_smem<k_e_warp<T, BY, 0, false, false>>(S);
-    set_smem<k_e_warp<T, BY, 0, true, false>>(S);
-    set_smem<k_e_warp<T, BY, 2, false, false>>(S);
-    set_smem<k_e_warp<T, BY, 2, true, false>>(S);
+    set_smem<k_e_warp<T, BY, 0, false>>(S);
+    set_smem<k_e_warp<T, BY, 0, true>>(S);
+    set_smem<k_e_warp<T, BY, 2, false>>(S);
+    set_smem<k_e_warp<T, BY, 2, true>>(S);
     set_smem<k_e_tma<T, BY, 0, false, true>>(SG);
     set_smem<k_e_tma<T, BY, 0, true, true>>(SG);
     set_smem<k_e_tma<T, BY, 1, false, true>>(SG);
@@ -305,10 +303,10 @@ int e_tma_by(const GridMaps &M, const FieldView<T> &f, const PmlView<T> &p, cons
                    : e_tma_launch<T, BY, 0, false, true>(M.t, f, p, D, G, kc, t.interior, err, s));
     }
     if (p.on)
-        return dl ? e_warp_launch<T, BY, 2, true, false>(M.e, f, p, G, kc, err, s)
-                  : e_warp_launch<T, BY, 2, false, false>(M.e, f, p, G, kc, err, s);
-    return dl ? e_warp_launch<T, BY, 0, true, false>(M.e, f, p, G, kc, err, s)
-              : e_warp_launch<T, BY, 0, false, false>(M.e, f, p, G, kc, err, s);
+        return dl ? e_warp_launch<T, BY, 2, true>(M.e, f, p, kc, err, s)
+                  : e_warp_launch<T, BY, 2, false>(M.e, f, p, kc, err, s);
+    return dl ? e_warp_launch<T, BY, 0, true>(M.e, f, p, kc, err, s)
+              : e_warp_launch<T, BY, 0, false>(M.e, f, p, kc, err, s);
 }
 
 template <typename T, int BY>

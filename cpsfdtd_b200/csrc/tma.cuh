@@ -24,7 +24,6 @@ struct TmaMaps {
 //   own   the swept side's, box 32 x BY x P x 3
 //   id    the IDs {px, ny+1, nz+1}, box 32 x BY x P
 //   tail  Ex and Ey of one plane, box 36 x (BY+1) x 1 x 2 (H sweep)
-//   gain  the gain words (as TmaMaps::gain)
 //   psi   by face, the side's two words, box 32 x BY x 1 x 2: x slabs {row
 //         words, ny+1, nz+1, 2}, y slabs {px, np+1, nz+1, 2}, z slabs {px, ny+1, np+1, 2}
 struct SweepMaps {
@@ -32,7 +31,6 @@ struct SweepMaps {
     CUtensorMap own[2];
     CUtensorMap id[2];
     CUtensorMap tail;
-    CUtensorMap gain;
     CUtensorMap psi[6];
 };
 

@@ -6,9 +6,8 @@
 // 16 lanes x 2 cells, 2 rows) and takes G = BY / RY such groups per plane.
 // Lane 0 keeps the planes ahead in flight with TMA loads into the warp's own
 // ring of stages of P planes each: one box per side for the three components
-// with their halo, one for the swept side's, one for the material IDs, one for
-// an FP32 E sweep's gain words and one per CPML axis the tile meets for its
-// two psi words.  One mbarrier per stage, no block barrier anywhere.
+// with their halo, one for the swept side's, one for the material IDs and one
+// per CPML axis the tile meets for its two psi words.  One mbarrier per stage, no block barrier anywhere.
 //
 // What bounds these sweeps is DRAM as long as the warps get through a plane
 // fast enough: 128 FP32 cells are 4.7 KB of traffic, 110 ns of an SM's share
@@ -91,23 +90,21 @@ struct WarpShape {
 };
 
 // The planes per stage of a tile: two where the stage holds fields alone, one
-// with psi or gain words (two such stages would not leave enough warps per SM)
+// with psi words (two such stages would not leave enough warps per SM)
 constexpr int kPlanes = 2;
 
 // Stage of P planes (offsets in bytes): halo components [3][P][BY+1][36], own
-// components [3][P][BY][32], IDs [P][BY][32], gain words [P][BY][15][32]; the
-// psi boxes [2][P][BY][32] of each axis follow.
-template <typename T, int BY, int P, bool G = false>
+// components [3][P][BY][32], IDs [P][BY][32]; the psi boxes [2][P][BY][32] of
+// each axis follow.
+template <typename T, int BY, int P>
 struct WarpStage {
     static constexpr int HROW = 36, HPL = HROW * (BY + 1), HC = P * HPL;  // elements: row, plane, component
     static constexpr int OPL = 32 * BY, OC = P * OPL;
     static constexpr int OWN = a128(3 * HC * (int)sizeof(T));
     static constexpr int ID = OWN + 3 * OC * (int)sizeof(T);
-    static constexpr int GAIN = ID + a128(OC);
-    static constexpr int GW = BY * kGainPersist * 32;                     // gain words of a plane
-    static constexpr int BYTES = GAIN + (G ? P * GW * 4 : 0);
+    static constexpr int BYTES = ID + a128(OC);
     static constexpr int PSI = 2 * OC * (int)sizeof(T);                   // one axis
-    static constexpr uint32_t TX = 3 * HC * sizeof(T) + 3 * OC * sizeof(T) + OC + (G ? P * GW * 4 : 0);
+    static constexpr uint32_t TX = 3 * HC * sizeof(T) + 3 * OC * sizeof(T) + OC;
     static constexpr uint32_t TAIL = 2 * HPL * sizeof(T);                 // Ex, Ey of one plane past the tile
 };
 
@@ -392,73 +389,13 @@ __device__ __forceinline__ void field_vst(T *p, const Vec<T> &a, unsigned wr)
     }
 }
 
-// four-level gain of the cells `on` of a vector (FP32, staged words): P -> E
-// -> N in gain_apply32's order of operations, one component at a time so that
-// no more than its four polarisation words are held; the new words go to the
-// dense state as whole vectors (the cells outside `on` carry their old words)
-__device__ __forceinline__ void gain_vec32(const GainView<float> &G, const float *ws, float *st, unsigned on,
-                                           Vec<float> &ex, Vec<float> &ey, Vec<float> &ez)
-{
-    using L = GainSite32;
-    const Vec<float> n1 = vld(ws + L::DN1 * 32), n2 = vld(ws + L::N2 * 32), n3 = vld(ws + L::N3 * 32);
-    float m0[4], dNa[4], dNb[4], sa[4], sb[4], s2[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        m0[q] = conserve_m0(n1.v[q], n2.v[q], n3.v[q]);  // FP64 conservation, FourLevelLaser.cpp:324
-        dNa[q] = (n2.v[q] - n1.v[q]) - 1.0f;
-        dNb[q] = (n3.v[q] - m0[q]) - 1.0f;
-    }
-#pragma unroll
-    for (int o = 0; o < 3; ++o) {
-        const int c = o == 0 ? 1 : o == 1 ? 0 : 2;
-        Vec<float> &ec = c == 0 ? ex : c == 1 ? ey : ez;
-        const Vec<float> pa = vld(ws + (L::PA + c) * 32), pa1 = vld(ws + (L::PA1 + c) * 32);
-        const Vec<float> pb = vld(ws + (L::PB + c) * 32), pb1 = vld(ws + (L::PB1 + c) * 32);
-        Vec<float> na, na1, nb, nb1;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const float E1 = ec.v[q];
-            float a, b, E;
-            gain_comp32(G.c, E1, dNa[q], dNb[q], pa.v[q], pa1.v[q], pb.v[q], pb1.v[q], a, b, E);
-            const float da = a - pa1.v[q], db = b - pb1.v[q], d2 = c == 1 ? a - pa.v[q] : da;
-            sa[q] = o == 0 ? rmul(E1, da) : rfma(E1, da, sa[q]);
-            sb[q] = o == 0 ? rmul(E1, db) : rfma(E1, db, sb[q]);
-            s2[q] = o == 0 ? rmul(E + E1, d2) : rfma(E + E1, d2, s2[q]);
-            const bool w = (on >> q) & 1u;
-            ec.v[q] = w ? E : E1;
-            na.v[q] = w ? a : pa.v[q];
-            na1.v[q] = w ? pa.v[q] : pa1.v[q];
-            nb.v[q] = w ? b : pb.v[q];
-            nb1.v[q] = w ? pb.v[q] : pb1.v[q];
-        }
-        vst(st + (L::PA + c) * kGainGroup, na);
-        vst(st + (L::PA1 + c) * kGainGroup, na1);
-        vst(st + (L::PB + c) * kGainGroup, nb);
-        vst(st + (L::PB1 + c) * kGainGroup, nb1);
-    }
-    Vec<float> r1, r2, r3;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        float a = n1.v[q], b = n2.v[q], e = n3.v[q];
-        gain_pops32(G.c, sa[q], sb[q], s2[q], m0[q], a, b, e);
-        const bool w = (on >> q) & 1u;
-        r1.v[q] = w ? a : n1.v[q];
-        r2.v[q] = w ? b : n2.v[q];
-        r3.v[q] = w ? e : n3.v[q];
-    }
-    vst(st + L::DN1 * kGainGroup, r1);
-    vst(st + L::N2 * kGainGroup, r2);
-    vst(st + L::N3 * kGainGroup, r3);
-}
-
 // Shared memory of a warp's ring (with 128 spare bytes to align it): two stages
-// of two planes, or three of one plane with gain words; either holds two
-// stages of a tile that meets a CPML slab on every axis.
-template <typename T, int BY, bool GAIN>
+// of two planes, or of one plane of a tile that meets a CPML slab on every axis.
+template <typename T, int BY>
 __host__ __device__ constexpr int warp_ring()
 {
-    constexpr int a = GAIN ? 3 * WarpStage<T, BY, 1, sizeof(T) == 4>::BYTES : 2 * WarpStage<T, BY, kPlanes>::BYTES;
-    constexpr int b = 2 * (WarpStage<T, BY, 1, GAIN && sizeof(T) == 4>::BYTES + 3 * WarpStage<T, BY, 1>::PSI);
+    constexpr int a = 2 * WarpStage<T, BY, kPlanes>::BYTES;
+    constexpr int b = 2 * (WarpStage<T, BY, 1>::BYTES + 3 * WarpStage<T, BY, 1>::PSI);
     return (a > b ? a : b) + 128;
 }
 
@@ -530,11 +467,11 @@ __device__ __forceinline__ Vec<T> along_i(const T *c, int i0, int nx)
 }
 
 // the psi boxes of a stage's planes from k; returns their bytes
-template <typename T, int BY, int P, bool G, bool ESIDE>
+template <typename T, int BY, int P, bool ESIDE>
 __device__ __forceinline__ uint32_t psi_bytes(const PmlView<T> &p, const Dims &d, const TilePsi &tp, int k, int &fz,
                                               int &sz)
 {
-    using L = WarpStage<T, BY, P, G>;
+    using L = WarpStage<T, BY, P>;
     fz = -1;
     if (tp.oz >= 0) fz = pair_face(p.np, d.nz, k, P, ESIDE, sz);
     return (tp.fx >= 0 ? L::PSI : 0) + (tp.fy >= 0 ? L::PSI : 0) + (fz >= 0 ? L::PSI : 0);
@@ -585,7 +522,7 @@ __device__ __forceinline__ bool h_warp_tile(const SweepMaps &M, const FieldView<
         }
         int fz = -1, sz = 0;
         uint32_t tx = L::TX;
-        if (PML) tx += psi_bytes<T, BY, P, false, false>(p, d, tp, k, fz, sz);
+        if (PML) tx += psi_bytes<T, BY, P, false>(p, d, tp, k, fz, sz);
         mbar_expect_tx(bar, tx + (m == 0 ? R.skew : 0u));
         tma_load_4d(b, &M.halo[P - 1], bar, x0, y0, k, 0);
         tma_load_4d(b + L::OWN, &M.own[P - 1], bar, x0, y0, k, 0);
@@ -719,13 +656,12 @@ __device__ __forceinline__ bool h_warp_tile(const SweepMaps &M, const FieldView<
 
 // E sweep of one tile by one warp: planes max(1, bz*kc) .. min(bz*kc+kc, nz)-1
 // (plane 0 is staged for its H alone).
-template <typename T, int BY, int P, bool PML, bool DL, bool GAIN>
-__device__ __forceinline__ bool e_warp_tile(const SweepMaps &M, const FieldView<T> &f, const PmlView<T> &p,
-                                            const GainView<T> &Gn, int kc, TileXYZ t, Ring &R, const Coef2<T> *tab)
+template <typename T, int BY, int P, bool PML, bool DL>
+__device__ __forceinline__ bool e_warp_tile(const SweepMaps &M, const FieldView<T> &f, const PmlView<T> &p, int kc,
+                                            TileXYZ t, Ring &R, const Coef2<T> *tab)
 {
-    static_assert(!GAIN || sizeof(T) == 4, "FP64 gain sweeps run the block-tile body");
-    static_assert(!(PML || GAIN) || P == 1, "psi and gain boxes hold one plane");
-    using L = WarpStage<T, BY, P, GAIN>;
+    static_assert(!PML || P == 1, "psi boxes hold one plane");
+    using L = WarpStage<T, BY, P>;
     using W = WarpShape<T>;
     constexpr int V = W::V, G = BY / W::RY;
     constexpr unsigned ALL = (1u << V) - 1;
@@ -746,13 +682,12 @@ __device__ __forceinline__ bool e_warp_tile(const SweepMaps &M, const FieldView<
         is = is + 1 == ns ? 0 : is + 1;
         int fz = -1, sz = 0;
         uint32_t tx = L::TX;
-        if (PML) tx += psi_bytes<T, BY, P, GAIN, true>(p, d, tp, k, fz, sz);
+        if (PML) tx += psi_bytes<T, BY, P, true>(p, d, tp, k, fz, sz);
         fence_proxy_async_smem();  // the stage's previous contents were read through the generic proxy
         mbar_expect_tx(bar, tx + (m == 0 ? R.skew : 0u));
         tma_load_4d(b, &M.halo[P - 1], bar, x0 - 4, y0 - 1, k, 0);
         tma_load_4d(b + L::OWN, &M.own[P - 1], bar, x0, y0, k, 0);
         tma_load_3d(b + L::ID, &M.id[P - 1], bar, x0, y0, k);
-        if (GAIN) tma_load_5d(b + L::GAIN, &M.gain, bar, 0, 0, t.bx, y0, k);
         if (PML) psi_issue(M, p, d, tp, b, bar, x0, y0, k, fz, sz);
     };
     if (lane == 0)
@@ -855,16 +790,6 @@ __device__ __forceinline__ bool e_warp_tile(const SweepMaps &M, const FieldView<
                         }
                     }
                     const int64_t w = w0 + (int64_t)(g * W::RY) * d.px;
-                    if constexpr (GAIN) {
-                        unsigned gain = 0;  // the gain list holds interior cells only
-#pragma unroll
-                        for (int q = 0; q < V; ++q)
-                            gain |= ((ids >> (8 * q)) & 255u) == (unsigned)Gn.gain_id ? 1u << q : 0u;
-                        gain &= row ? act : 0u;
-                        if (gain)
-                            gain_vec32(Gn, (const float *)(b + L::GAIN) + u * L::GW + (g * W::RY + ly) * kGainPersist * 32 + lx * V,
-                                       Gn.state + gain_dense_index(w), gain, ex, ey, ez);
-                    }
                     if (PML) {
                         if (p.literal) bE = splat(p.cpmlE);
                         pml_vec<T, true>(p, d, tp, b + (u * L::OPL + o) * (int)sizeof(T), L::OC, px, ry[g], fz,
