@@ -624,8 +624,8 @@ cps_status check_device_error(cps_grid *g)
     return CPS_OK;
 }
 
-// whether a TF/SF target or a source may lie in a CPML slab (E slabs reach
-// index np, one further than H slabs; H targets lie one cell outside the box)
+// whether a TF/SF target may lie in a CPML slab (E slabs reach index np, one
+// further than H slabs; H targets lie one cell outside the box)
 bool tfsf_meets_pml(const cps_grid *g)
 {
     for (int f = 0; f < 6; ++f)
@@ -633,6 +633,9 @@ bool tfsf_meets_pml(const cps_grid *g)
     return false;
 }
 
+// A source adds to its component between the E bulk update and the E CPML
+// routine.  That routine reads E and H at its cell and H one cell below on each
+// axis, so an H source also reaches it from one cell in front of a far slab.
 bool sources_meet_pml(const cps_grid *g)
 {
     const Dims &d = g->d;
@@ -640,8 +643,9 @@ bool sources_meet_pml(const cps_grid *g)
     for (const Src &s : g->src) {
         const int k = (int)(s.idx / d.pxy), j = (int)((s.idx - k * d.pxy) / d.px);
         const int at[3] = {(int)(s.idx - k * d.pxy - (int64_t)j * d.px), j, k};
+        const int below = s.comp >= CPS_HX ? 1 : 0;
         for (int a = 0; a < 3; ++a)
-            if (at[a] <= g->pml.npml[2 * a] || at[a] >= n[a] - g->pml.npml[2 * a + 1]) return true;
+            if (at[a] <= g->pml.npml[2 * a] || at[a] >= n[a] - g->pml.npml[2 * a + 1] - below) return true;
     }
     return false;
 }
