@@ -34,7 +34,8 @@ struct GridSig {
     int64_t step;
     const void *f0, *dl, *gain, *st, *q, *tg0, *tg1, *srcw, *ring0;
     int64_t dl_n, g_n;
-    int nports, nsrc, ntg0, ntg1, pml, by, kc;
+    int nports, nsrc, ntg0, ntg1, pml, by;
+    int rows, kc, kch, kcg, fixed;  // the grid's tile shape
     int64_t nfreq_sum;
     bool operator==(const GridSig &o) const { return memcmp(this, &o, sizeof(GridSig)) == 0; }
 };
@@ -50,7 +51,8 @@ GridSig signature(const cps_grid *g)
     s.dl_n = g->dl_on ? g->dl_n : -1; s.g_n = g->gain_on ? g->g_n : -1;
     s.nports = (int)g->ports.size(); s.nsrc = (int)g->src.size();
     s.ntg0 = g->tfsf_on ? g->ntg[0] : -1; s.ntg1 = g->tfsf_on ? g->ntg[1] : -1;
-    s.pml = g->pml_on; s.by = g->tma_by; s.kc = g->shape.kc;
+    s.pml = g->pml_on; s.by = g->tma_by;
+    s.rows = g->shape.by; s.kc = g->shape.kc; s.kch = g->shape.kch; s.kcg = g->shape.kcg; s.fixed = g->shape.fixed;
     for (const PortState &P : g->ports) s.nfreq_sum += P.nfreq * 7 + P.npts;
     return s;
 }
@@ -383,7 +385,8 @@ cps_status rebuild_T(cps_batch *b)
 // Tile shape of a member's own sweep launches: the batch's when the caller set
 // it, the grid's own in a one-grid batch; else the grid's planes as they are
 // (members run beside one another, so a small one need not fill the device)
-// and the batch's for the E sweep with gain.
+// and the batch's for the E sweep with gain.  The rows are the batch's always:
+// the tensor maps are encoded for them when the tables are made.
 FusedShape member_shape(const cps_batch *b, const cps_grid *g)
 {
     FusedShape sh = g->shape;
@@ -394,6 +397,7 @@ FusedShape member_shape(const cps_batch *b, const cps_grid *g)
         sh.kcg = b->kc;
         sh.fixed = true;
     }
+    sh.by = b->by;
     return sh;
 }
 

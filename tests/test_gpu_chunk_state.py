@@ -1,0 +1,98 @@
+"""Fused steps as replayed chunks after something else has touched the grid:
+port samples taken outside the step, media set again, tiles set again, the
+wait's test setting, and short calls.  Chunks and single launches do the same
+operations on every cell and sample, so results are equal bit for bit."""
+import time
+
+import numpy as np
+import pytest
+
+from cpsfdtd_b200 import decks
+from test_gpu_step_paths import _noise, _same, _state
+
+pytestmark = pytest.mark.gpu
+
+
+def _pair(dk, prec):
+    """the grid in chunks and the same grid in single launches"""
+    import cpsfdtd_b200 as cps
+    a, b = cps.Grid.from_deck(dk, prec), cps.Grid.from_deck(dk, prec)
+    b.set_chunked(False)
+    for g in (a, b):
+        _noise(g, dk, 11)
+    return a, b
+
+
+@pytest.mark.parametrize("deck", ["dispersive", "laser"])
+@pytest.mark.parametrize("prec", [0, 1], ids=["fp64", "fp32"])
+def test_tile_set_on_a_batch_member_between_steps(prec, deck):
+    """A member's tile set while it is in a batch whose tables are made: the
+    batch's rows hold for its own sweeps (the tensor maps' rows), in chunks
+    launched directly (a new length) and replayed (a length that comes again)."""
+    import cpsfdtd_b200 as cps
+    mk = {"dispersive": lambda n: decks.config2(n=n, steps=1, nfreq=3),
+          "laser": lambda n: decks.config4_member(n, n - 3, n - 5, seed=3, steps=1, nfreq=2)}[deck]
+    dks = [mk(40), mk(53)]
+    got = []
+    for tiles in (False, True):
+        gs = [cps.Grid.from_deck(dk, prec) for dk in dks]
+        for g, dk in zip(gs, dks):
+            _noise(g, dk, 12)
+        bt = cps.Batch(prec)
+        for g in gs:
+            bt.add(g)
+        for rows, planes in ((8, 8), (4, 8), (8, 16), (4, 2), (8, 1)):
+            for n in (7, 12, 12):
+                bt.step(n)
+                if tiles:
+                    gs[0].set_tile(rows, planes)
+        bt.sync()
+        got.append([_state(g) for g in gs])
+        for g in gs:
+            bt.remove(g)
+        bt.close()
+    for x, y in zip(*got):
+        _same(x, y)
+
+
+@pytest.mark.parametrize("prec", [0, 1], ids=["fp64", "fp32"])
+def test_tile_set_on_a_chunked_grid(prec):
+    """The grid's own chunks follow its tile: rows and planes, the default's own
+    among them."""
+    import cpsfdtd_b200 as cps
+    a, b = _pair(decks.config2(n=45, steps=1, nfreq=3), prec)
+    for g in (a, b):
+        g.step(192, cps.FUSED)
+        for rows, planes in ((4, 8), (8, 8), (8, 1), (4, 64), (16, 4), (4, 8)):
+            g.set_tile(rows, planes)
+            g.step(64, cps.FUSED)
+    _same(_state(a), _state(b))
+
+
+@pytest.mark.parametrize("prec", [0, 1], ids=["fp64", "fp32"])
+def test_steps_alone_between_batch_steps(prec):
+    """A member's own long calls (its own chunks) between the batch's."""
+    import cpsfdtd_b200 as cps
+    dks = [decks.config2(n=40, steps=1, nfreq=3), decks.config2(n=49, steps=1, nfreq=2)]
+    out = []
+    for alone in (False, True):
+        gs = [cps.Grid.from_deck(dk, prec) for dk in dks]
+        for g, dk in zip(gs, dks):
+            _noise(g, dk, 13)
+        bt = cps.Batch(prec)
+        for g in gs:
+            bt.add(g)
+        for n in (64, 40, 64, 5, 64):
+            bt.step(n)
+            if alone:
+                gs[0].step(70, cps.FUSED)
+                gs[0].step(3, cps.FUSED)
+        bt.sync()
+        if not alone:
+            gs[0].step(5 * 73, cps.FUSED)
+        out.append([_state(g) for g in gs])
+        for g in gs:
+            bt.remove(g)
+        bt.close()
+    for x, y in zip(*out):
+        _same(x, y)
