@@ -250,9 +250,6 @@ cps_status rebuild_T(cps_batch *b)
         if ((s = ensure_sources(g))) return s;
         if (g->shape.by != by) g->shape.by = by;
         if ((s = ensure_tma(g))) return s;
-        // fold samples left in the rings by one-grid stepping
-        for (PortState &P : g->ports)
-            if (P.fill > 0 && P.nfreq > 0 && (s = flush_dft(g, P))) return s;
         CK(cudaStreamSynchronize(g->stream));
         BatchGrid<T> &B = hg[gi];
         memset((void *)&B, 0, sizeof(B));
@@ -532,11 +529,13 @@ cps_status step_batch_T(cps_batch *b, int nsteps)
         if ((s = rebuild_T<T>(b))) return s;
         moved.clear();
     }
-    for (size_t q : moved) {
-        cps_grid *g = b->grids[q];
-        // fold samples left in the rings by one-grid stepping
+    // fold samples that one-grid steps or single routines left in the rings: the
+    // chunk fills them from the start
+    for (cps_grid *g : b->grids)
         for (PortState &P : g->ports)
             if (P.fill > 0 && P.nfreq > 0 && (s = flush_dft(g, P))) return s;
+    for (size_t q : moved) {
+        cps_grid *g = b->grids[q];
         launch_set_step_batch<T>((BatchGrid<T> *)b->d_grids, (int)q, g->step, b->stream);
         b->sigs[q].step = g->step;
     }

@@ -96,3 +96,18 @@ def test_steps_alone_between_batch_steps(prec):
         bt.close()
     for x, y in zip(*out):
         _same(x, y)
+
+
+@pytest.mark.parametrize("prec", [0, 1], ids=["fp64", "fp32"])
+def test_port_samples_between_chunks_are_kept(prec):
+    import cpsfdtd_b200 as cps
+    dk = decks.config2(n=41, steps=1, nfreq=3)
+    a, b = _pair(dk, prec)
+    for g in (a, b):
+        g.step(64, cps.FUSED)
+        n = g.get_step()
+        for s in range(n, n + 64):  # a whole ring, the grid's own step number unmoved
+            for p in range(len(g.ports)):
+                g.op("port_sample", p, s)
+        g.step(64, cps.FUSED)
+    _same(_state(a), _state(b))
