@@ -37,6 +37,7 @@ struct GridSig {
     int nports, nsrc, ntg0, ntg1, pml, by;
     int rows, kc, kch, kcg, fixed;  // the grid's tile shape
     int64_t nfreq_sum;
+    double ce_disp;  // of the CPML view, which chunks hold by value
     bool operator==(const GridSig &o) const { return memcmp(this, &o, sizeof(GridSig)) == 0; }
 };
 
@@ -54,6 +55,7 @@ GridSig signature(const cps_grid *g)
     s.pml = g->pml_on; s.by = g->tma_by;
     s.rows = g->shape.by; s.kc = g->shape.kc; s.kch = g->shape.kch; s.kcg = g->shape.kcg; s.fixed = g->shape.fixed;
     for (const PortState &P : g->ports) s.nfreq_sum += P.nfreq * 7 + P.npts;
+    s.ce_disp = pml_view<double>(g).ce_disp;
     return s;
 }
 

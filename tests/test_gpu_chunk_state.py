@@ -111,3 +111,25 @@ def test_port_samples_between_chunks_are_kept(prec):
                 g.op("port_sample", p, s)
         g.step(64, cps.FUSED)
     _same(_state(a), _state(b))
+
+
+@pytest.mark.parametrize("prec", [0, 1], ids=["fp64", "fp32"])
+def test_media_set_again_reach_the_chunks(prec):
+    """ID 2 without the Drude-Lorentz module keeps its E bulk update out, and its
+    CPML term takes the medium's curl coefficient: set between two chunks of
+    one length, the second of them a replay."""
+    import cpsfdtd_b200 as cps
+    d = 10e-9
+    dk = decks.Deck(40, 37, 33, d, d, d)
+    dk.media = [(1.0, 1.0, 0.0, 0.0), (2.25, 1.0, 0.0, 0.0), (2.0, 1.0, 0.0, 0.0)]
+    ids = np.zeros(dk.shape3, dtype=np.uint8)
+    ids[2:4, 10:14, 12:15] = 2  # in the x slab; such cells only sum psi terms: few steps
+    dk.ids = ids
+    dk.pml = decks.pml_params(5)
+    a, b = _pair(dk, prec)
+    for g in (a, b):
+        for _ in range(3):
+            g.step(32, cps.FUSED)
+        g.set_media([(1.0, 1.0, 0.0, 0.0), (2.25, 1.0, 0.0, 0.0), (5.0, 1.0, 0.0, 0.0)])
+        g.step(32, cps.FUSED)
+    _same(_state(a), _state(b))
