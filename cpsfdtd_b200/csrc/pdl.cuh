@@ -11,8 +11,9 @@
 // successor only take places that the predecessor's blocks, all of them
 // scheduled by then, leave free.  Every block waits, one without work too: a
 // kernel whose blocks all left early would pass for its predecessors' end with
-// the next one.  Without
-// the launch attribute both calls do nothing.
+// the next one.  What a predecessor writes is read with plain loads: the
+// non-coherent load is for words unwritten while the kernel lives, and the wait
+// does not hold it back.  Without the launch attribute both calls do nothing.
 //
 // Launched early: the sweeps, the plain path's bulk updates, and the injection,
 // source and gather kernels of single steps (us per step, before and after:

@@ -168,25 +168,27 @@ struct PsiRegs {
     T x0, x1, y0, y1, z0, z1;
 };
 
-// E-side psi of plane k for a column (slab membership as in pml_e_cell)
+// E-side psi of plane k for a column (slab membership as in pml_e_cell).  Plain
+// loads here and in psi_load_h: a sweep is launched while its predecessor still
+// writes these words, and only plain loads stay behind its wait (pdl.cuh).
 template <typename T>
 __device__ __forceinline__ void psi_load_e(const PmlView<T> &p, const Dims &d, const ColPml<T> &c, int i, int j, int k,
                                            PsiRegs<T> &r)
 {
     if (c.fx >= 0) {
         const int64_t q = ((int64_t)k * (d.ny + 1) + j) * psi_xw(p.np[c.fx]) + c.sxl;
-        r.x0 = __ldg(p.qe[c.fx][0] + q); r.x1 = __ldg(p.qe[c.fx][1] + q);
+        r.x0 = p.qe[c.fx][0][q]; r.x1 = p.qe[c.fx][1][q];
     }
     if (c.fy >= 0) {
         const int64_t q = ((int64_t)k * (p.np[c.fy] + 1) + c.syl) * d.px + i;
-        r.y0 = __ldg(p.qe[c.fy][0] + q); r.y1 = __ldg(p.qe[c.fy][1] + q);
+        r.y0 = p.qe[c.fy][0][q]; r.y1 = p.qe[c.fy][1][q];
     }
     int fz = -1, szl = 0;
     if (k <= p.np[kFZ1]) { fz = kFZ1; szl = k; }
     else if (k >= d.nz - p.np[kFZ2]) { fz = kFZ2; szl = k - (d.nz - p.np[kFZ2]); }
     if (fz >= 0) {
         const int64_t q = ((int64_t)szl * (d.ny + 1) + j) * d.px + i;
-        r.z0 = __ldg(p.qe[fz][0] + q); r.z1 = __ldg(p.qe[fz][1] + q);
+        r.z0 = p.qe[fz][0][q]; r.z1 = p.qe[fz][1][q];
     }
 }
 
@@ -197,18 +199,18 @@ __device__ __forceinline__ void psi_load_h(const PmlView<T> &p, const Dims &d, c
 {
     if (c.fx >= 0) {
         const int64_t q = ((int64_t)k * (d.ny + 1) + j) * psi_xw(p.np[c.fx]) + c.sxl;
-        r.x0 = __ldg(p.qh[c.fx][0] + q); r.x1 = __ldg(p.qh[c.fx][1] + q);
+        r.x0 = p.qh[c.fx][0][q]; r.x1 = p.qh[c.fx][1][q];
     }
     if (c.fy >= 0) {
         const int64_t q = ((int64_t)k * (p.np[c.fy] + 1) + c.syl) * d.px + i;
-        r.y0 = __ldg(p.qh[c.fy][0] + q); r.y1 = __ldg(p.qh[c.fy][1] + q);
+        r.y0 = p.qh[c.fy][0][q]; r.y1 = p.qh[c.fy][1][q];
     }
     int fz = -1, szl = 0;
     if (k < p.np[kFZ1]) { fz = kFZ1; szl = k; }
     else if (k >= d.nz - p.np[kFZ2]) { fz = kFZ2; szl = k - (d.nz - p.np[kFZ2]); }
     if (fz >= 0) {
         const int64_t q = ((int64_t)szl * (d.ny + 1) + j) * d.px + i;
-        r.z0 = __ldg(p.qh[fz][0] + q); r.z1 = __ldg(p.qh[fz][1] + q);
+        r.z0 = p.qh[fz][0][q]; r.z1 = p.qh[fz][1][q];
     }
 }
 

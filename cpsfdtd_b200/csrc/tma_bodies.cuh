@@ -219,8 +219,8 @@ __device__ __forceinline__ bool e_tma_body(const TmaMaps &M, const FieldView<T> 
     T hxm = 0, hym = 0;
     if (rowok) {
         const int64_t gm = d.idx(i, j, k0 - 1);
-        hxm = __ldg(&f.Hx[gm]);
-        hym = __ldg(&f.Hy[gm]);
+        hxm = f.Hx[gm];
+        hym = f.Hy[gm];
     }
     // psi two planes ahead: qc (plane k), qn (k+1), loads for k+2 issued at plane k
     // (one plane ahead, in shared slots, beside an FP64 cell's gain words)

@@ -50,19 +50,6 @@ __device__ __forceinline__ void vst(T *p, const Vec<T> &a)
 {
     *reinterpret_cast<Vec<T> *>(p) = a;
 }
-// global vector load from L2 (the word may have been written by another SM in
-// this launch)
-__device__ __forceinline__ Vec<float> vldcg(const float *p)
-{
-    const float4 a = __ldcg(reinterpret_cast<const float4 *>(p));
-    return Vec<float>{{a.x, a.y, a.z, a.w}};
-}
-__device__ __forceinline__ Vec<double> vldcg(const double *p)
-{
-    const double2 a = __ldcg(reinterpret_cast<const double2 *>(p));
-    return Vec<double>{{a.x, a.y}};
-}
-
 // tile q of a grid of nbx x nby tiles per plane row of tiles, x fastest
 __device__ __forceinline__ TileXYZ grid_tile(int q, int nbx, int nby)
 {
@@ -705,8 +692,8 @@ __device__ __forceinline__ bool e_warp_tile(const SweepMaps &M, const FieldView<
         cExz[g] = sv.cExz[j];
         cEzx[g] = sv.cEzx[j];
         const int64_t w = d.idx(i0, j, max(k0 - 1, 0));
-        hxm[g] = vldcg(f.Hx + w);
-        hym[g] = vldcg(f.Hy + w);
+        hxm[g] = vld(f.Hx + w);
+        hym[g] = vld(f.Hy + w);
         if (PML) {
             ry[g].f = slab_face(p.np, kFY1, d.ny, j, true, ry[g].s);
             if (ry[g].f >= 0) {
