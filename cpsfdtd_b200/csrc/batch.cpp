@@ -436,6 +436,9 @@ int64_t enqueue_chunk(cps_batch *b, int S)
     const BatchPort<T> *P = (const BatchPort<T> *)b->d_ports;
     cudaStream_t st = b->stream;
     int64_t n = 0;
+    // a grid's internal batch reports to the grid's own error word, which also
+    // holds the waits' test setting
+    int *const err = b->grid_tiles ? b->grids[0]->d_err : b->d_err;
     for (int s = 0; s < S; ++s) {
         // one grid: its pointers as kernel parameters, not through the tables
         auto inject = [&](int side) {
@@ -444,20 +447,20 @@ int64_t enqueue_chunk(cps_batch *b, int S)
             else
                 launch_inject_batch<T>(G, b->d_inj[side], b->ninj[side], side, s, st);
         };
-        launch_h_batch<T>(G, b->d_tiles[kHInt], b->ntiles[kHInt], b->nblocks[kHInt], b->by, false, b->d_err, st);
-        launch_h_batch<T>(G, b->d_tiles[kHPml], b->ntiles[kHPml], b->nblocks[kHPml], b->by, true, b->d_err, st);
+        launch_h_batch<T>(G, b->d_tiles[kHInt], b->ntiles[kHInt], b->nblocks[kHInt], b->by, false, err, st);
+        launch_h_batch<T>(G, b->d_tiles[kHPml], b->ntiles[kHPml], b->nblocks[kHPml], b->by, true, err, st);
         per_member(b, [&](int gi, cudaStream_t ms) {
             const cps_grid *g = b->grids[gi];
-            n += launch_h_tma<T>(g->tma, field_view<T>(g), pml_view<T>(g), member_shape(b, g), b->d_err, ms);
+            n += launch_h_tma<T>(g->tma, field_view<T>(g), pml_view<T>(g), member_shape(b, g), err, ms);
         });
         inject(1);
         for (int c = 0; c < 8; ++c)
-            launch_e_batch<T>(G, b->d_tiles[kE0 + c], b->ntiles[kE0 + c], b->nblocks[kE0 + c], b->by, c, b->d_err, st);
+            launch_e_batch<T>(G, b->d_tiles[kE0 + c], b->ntiles[kE0 + c], b->nblocks[kE0 + c], b->by, c, err, st);
         launch_dl_batch<T>(G, b->d_dl, b->ndl, st);
         per_member(b, [&](int gi, cudaStream_t ms) {
             const cps_grid *g = b->grids[gi];
             n += launch_e_tma<T>(g->tma, field_view<T>(g), pml_view<T>(g), dl_view<T>(g), gain_view<T>(g),
-                            member_shape(b, g), b->d_err, ms, &g->lane);
+                            member_shape(b, g), err, ms, &g->lane);
         });
         inject(0);
         launch_sources_batch<T>(G, b->d_src, b->nsrc, s, st);
@@ -620,14 +623,6 @@ void cps::batch_use_grid_tiles(cps_batch *b)
     if (b->tile_set) b->dirty = true;  // captured chunks launch the per-member sweeps with the tiling
     b->tile_set = false;
     b->grid_tiles = true;
-}
-
-// clears a batch's device error word (the grid reset of a grid stepped
-// through its internal one-grid batch)
-cps_status cps::batch_clear_error(cps_batch *b)
-{
-    if (b->d_err) CK(cudaMemsetAsync(b->d_err, 0, sizeof(int), b->stream));
-    return CPS_OK;
 }
 
 // ================================================================ C ABI

@@ -925,8 +925,9 @@ extern "C" cps_status cps_synchronize(cps_grid *g)
     REQUIRE(g, CPS_E_INVALID, "NULL grid");
     FLUSH_RECORDED(g);
     if (g->solo) {
-        cps_status s = cps_batch_synchronize(g->solo);
-        if (s) return s;
+        void *chunks = nullptr;
+        cps_batch_get_stream(g->solo, &chunks);
+        CK(cudaStreamSynchronize((cudaStream_t)chunks));
     }
     CK(cudaStreamSynchronize(g->stream));
     return check_device_error(g);
@@ -2072,10 +2073,6 @@ extern "C" cps_status cps_grid_reset(cps_grid *g, int64_t n0)
     }
     // a sweep that gave up left the state incomplete; the reset state is whole again
     CK(cudaMemsetAsync(g->d_err, 0, sizeof(int), g->stream));
-    if (g->solo) {
-        cps_status s = batch_clear_error(g->solo);
-        if (s) return s;
-    }
     g->step = n0;
     CK(cudaStreamSynchronize(g->stream));
     return CPS_OK;

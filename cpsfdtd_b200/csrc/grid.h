@@ -360,8 +360,6 @@ inline ThreeView three_view(const cps_grid *g)
     return v;
 }
 
-// clears the device error word of a batch (batch.cpp)
-cps_status batch_clear_error(cps_batch *b);
 // per-member launches of a batch take each grid's own tile shape
 void batch_use_grid_tiles(cps_batch *b);
 

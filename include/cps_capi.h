@@ -354,8 +354,8 @@ CPS_API cps_status cps_grid_reset(cps_grid *g, int64_t n0);
 /* test setting for the bounded device waits (no reference counterpart; the
  * reference has no failure handling, main.cpp:68-85): with extra_bytes > 0
  * (at most 4096) the first plane of every tile of this grid's own TMA sweeps
- * (cps_step FUSED below the chunked size, cps_op_* and recorded steps)
- * expects that many more bytes than its loads bring, so each block's wait
+ * (cps_step FUSED, in chunks or not, cps_op_* and recorded steps; not those a
+ * cps_batch launches) expects that many more bytes than its loads bring, so each block's wait
  * runs out after its limit (about a second) and the step reports
  * CPS_E_TIMEOUT at the next synchronisation, with no fault and the context
  * intact.  0 (the default) restores normal operation; cps_grid_reset then

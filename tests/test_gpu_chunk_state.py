@@ -133,3 +133,34 @@ def test_media_set_again_reach_the_chunks(prec):
         g.set_media([(1.0, 1.0, 0.0, 0.0), (2.25, 1.0, 0.0, 0.0), (5.0, 1.0, 0.0, 0.0)])
         g.step(32, cps.FUSED)
     _same(_state(a), _state(b))
+
+
+@pytest.mark.parametrize("prec", [0, 1], ids=["fp64", "fp32"])
+def test_wait_setting_reaches_the_chunks(prec):
+    """A chunk gives up its waits, says so, and the grid steps as a fresh one after
+    a reset (no fault is involved: every wait is bounded and every copy lands).
+    A grid of 4 Mi cells steps in chunks always; tiles of all its planes are
+    few enough to wait at the same time."""
+    import cpsfdtd_b200 as cps
+    d = 10e-9
+    dk = decks.Deck(512, 128, 65, d, d, d)
+    dk.sources = [(decks.COMP["Ez"], 250, 64, 30, decks.gaussian_sine(400, dk.dt, 600e-9, 5e-16, 7e-16))]
+    g, ref = cps.Grid.from_deck(dk, prec), cps.Grid.from_deck(dk, prec)
+    for q in (g, ref):
+        q.set_tile(8, 128)
+    g.step(64, cps.FUSED)
+    g.sync()
+    g.set_wait_skew(256)
+    t0 = time.perf_counter()
+    g.step(1, cps.FUSED)
+    with pytest.raises(cps.CpsError) as ex:
+        g.sync()
+    assert ex.value.code == cps.CPS_E_TIMEOUT
+    assert time.perf_counter() - t0 < 30.0
+    g.set_wait_skew(0)
+    g.reset(dk.n0)
+    for q in (g, ref):
+        q.step(64, cps.FUSED)
+        q.sync()
+    for c in range(6):
+        assert np.array_equal(g.field(c), ref.field(c))
