@@ -1634,11 +1634,22 @@ namespace {
 constexpr int64_t kSoloCells = 4 << 20;
 constexpr int kSoloSteps = 32;
 
+// whether the caller is capturing the grid's stream: a chunk has a stream and
+// graphs of its own, which cannot be made inside another capture
+bool capturing(const cps_grid *g)
+{
+    cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(g->stream, &c) == cudaSuccess) return c != cudaStreamCaptureStatusNone;
+    cudaGetLastError();
+    return true;
+}
+
 bool solo_eligible(const cps_grid *g, int nsteps)
 {
     return g->chunked && g->timing_stride == 0 && g->sweep_mode == 0 && !g->three_on &&
            (g->shape.by == 4 || g->shape.by == 8) && g->d.px >= 64 && g->d.ny >= 8 && g->d.nz >= 2 &&
-           (g->solo || nsteps >= kSoloSteps || (int64_t)g->d.nx * g->d.ny * g->d.nz >= kSoloCells);
+           (g->solo || nsteps >= kSoloSteps || (int64_t)g->d.nx * g->d.ny * g->d.nz >= kSoloCells) &&
+           !capturing(g);
 }
 
 cps_status solo_step(cps_grid *g, int32_t nsteps)
