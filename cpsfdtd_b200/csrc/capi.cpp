@@ -15,6 +15,7 @@
 #include <thread>
 #include <vector>
 
+#include "batch.h"
 #include "grid.h"
 #include "tfsf_csr.h"
 
@@ -1626,13 +1627,33 @@ namespace {
 // Fused steps run as chunks of a one-grid batch: the batch launches the grid's
 // sweeps inside CUDA-graph-replayed chunks and the rest of the step in batched
 // launches, with results equal to the direct launches.  On a small grid a step
-// is a few microseconds of kernels, far less than its launches take to issue
-// (48^3: 24 us a step launched directly, 12 replayed), on a large one the gaps
-// between them still show (256^3: 2.5 %).  Making the batch's tables takes about
-// the time of 16 direct small steps, so shorter calls on a small grid that has
-// no tables yet are launched directly.
+// is a few microseconds of kernels, less than its launches take to issue (48^3
+// dielectric 12.9 us a step launched directly, 11.1 replayed; 41^3 dispersive
+// 27 and 21), on a large one the gaps between them still show (256^3: 2.5 %).
+// Making the batch's tables takes about the time of 16 direct small steps, so
+// shorter calls on a small grid that has no tables yet are launched directly.
 constexpr int64_t kSoloCells = 4 << 20;
 constexpr int kSoloSteps = 32;
+
+// Whether replaying n steps of a small grid saves more than the chunk costs.  A
+// chunk folds the ports' DFT at its end, where direct steps do once in 64
+// samples; a fold takes 15 us and the accumulators' round trip at 6 TB/s, a
+// chunk's start 8 us.  A replayed step saves 1.3 us at least, 3 where the
+// Drude-Lorentz pass runs beside its E sweep on a second stream.  Measured, us a
+// step direct and in chunks: 48^3 dielectric, 1 step 14.4 and 16.5, 10 steps
+// 13.3 and 11.5; 96^3 laser, 1 step 43.9 and 58.3, 24 steps 43.8 and 41.7; 128^3
+// dispersive (157 MB of accumulators), 1 step 69 and 111, 10 steps 68.6 and
+// 68.8, 24 steps 69.0 and 66.3; with 1255 MB in FP64, 32 steps 133.1 and 135.3,
+// 48 steps 133.5 and 132.1.
+bool chunk_pays(const cps_grid *g, int n)
+{
+    if (n >= kMaxRing) return true;
+    double bytes = 0, fold = 0;
+    for (const PortState &P : g->ports)
+        if (P.nfreq > 0) bytes += 32.0 * P.ncomp * P.nfreq * P.npts, fold = 15.0;
+    fold += bytes / 6e6;
+    return (g->dl_on ? 3.0 : 1.3) * n >= 8.0 + fold * (1.0 - n / (double)kMaxRing);
+}
 
 // whether the caller is capturing the grid's stream: a chunk has a stream and
 // graphs of its own, which cannot be made inside another capture
@@ -1648,7 +1669,8 @@ bool solo_eligible(const cps_grid *g, int nsteps)
 {
     return g->chunked && g->timing_stride == 0 && g->sweep_mode == 0 && !g->three_on &&
            (g->shape.by == 4 || g->shape.by == 8) && g->d.px >= 64 && g->d.ny >= 8 && g->d.nz >= 2 &&
-           (g->solo || nsteps >= kSoloSteps || (int64_t)g->d.nx * g->d.ny * g->d.nz >= kSoloCells) &&
+           ((int64_t)g->d.nx * g->d.ny * g->d.nz >= kSoloCells ||
+            ((g->solo || nsteps >= kSoloSteps) && chunk_pays(g, nsteps))) &&
            !capturing(g);
 }
 

@@ -164,3 +164,21 @@ def test_wait_setting_reaches_the_chunks(prec):
         q.sync()
     for c in range(6):
         assert np.array_equal(g.field(c), ref.field(c))
+
+
+def test_short_calls_fold_the_ports_once_a_ring():
+    """A loop of single steps on a small grid with a port DFT launches what it does
+    on a grid without chunks: the contraction runs once in 64 samples, not once a
+    call."""
+    import cpsfdtd_b200 as cps
+    dk = decks.config2(n=41, steps=1, nfreq=3)
+    a, b = _pair(dk, cps.FP32)
+    n = []
+    for g in (a, b):
+        g.step(64, cps.FUSED)
+        n0 = g.launches()
+        for _ in range(130):
+            g.step(1, cps.FUSED)
+        n.append(g.launches() - n0)
+    assert n[0] <= n[1] + 4, n
+    _same(_state(a), _state(b))
