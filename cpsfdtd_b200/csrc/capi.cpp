@@ -639,15 +639,12 @@ bool tfsf_meets_pml(const cps_grid *g)
 // axis, so an H source also reaches it from one cell in front of a far slab.
 bool sources_meet_pml(const cps_grid *g)
 {
-    const Dims &d = g->d;
-    const int n[3] = {d.nx, d.ny, d.nz};
-    for (const Src &s : g->src) {
-        const int k = (int)(s.idx / d.pxy), j = (int)((s.idx - k * d.pxy) / d.px);
-        const int at[3] = {(int)(s.idx - k * d.pxy - (int64_t)j * d.px), j, k};
-        const int below = s.comp >= CPS_HX ? 1 : 0;
+    const int n[3] = {g->d.nx, g->d.ny, g->d.nz};
+    for (int side = 0; side < 2; ++side)  // E sources, H sources
         for (int a = 0; a < 3; ++a)
-            if (at[a] <= g->pml.npml[2 * a] || at[a] >= n[a] - g->pml.npml[2 * a + 1] - below) return true;
-    }
+            if (g->src_lo[side][a] <= g->pml.npml[2 * a] ||
+                g->src_hi[side][a] >= n[a] - g->pml.npml[2 * a + 1] - side)
+                return true;
     return false;
 }
 
@@ -1474,6 +1471,11 @@ extern "C" cps_status cps_source_add(cps_grid *g, int32_t comp, int32_t i, int32
     s.comp = comp; s.idx = g->d.idx(i, j, k); s.wave.assign(wave, wave + nwave);
     g->src.push_back(s);
     g->src_dirty = true;
+    const int side = comp >= CPS_HX ? 1 : 0, at[3] = {i, j, k};
+    for (int a = 0; a < 3; ++a) {
+        g->src_lo[side][a] = std::min(g->src_lo[side][a], at[a]);
+        g->src_hi[side][a] = std::max(g->src_hi[side][a], at[a]);
+    }
     return CPS_OK;
 }
 

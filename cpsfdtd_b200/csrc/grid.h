@@ -2,6 +2,7 @@
 // the C ABI (capi.cpp) and the batched engine (batch.cpp).
 #pragma once
 
+#include <stdint.h>
 #include <string.h>
 
 #include <string>
@@ -139,6 +140,9 @@ struct cps_grid {
     int ntg[2] = {0, 0};
     // sources
     std::vector<Src> src;
+    // box of the E sources' and of the H sources' points (empty: lo > hi)
+    int src_lo[2][3] = {{INT32_MAX, INT32_MAX, INT32_MAX}, {INT32_MAX, INT32_MAX, INT32_MAX}};
+    int src_hi[2][3] = {{-1, -1, -1}, {-1, -1, -1}};
     int64_t *d_src_idx = nullptr;
     int32_t *d_src_comp = nullptr, *d_src_off = nullptr, *d_src_len = nullptr;
     double *d_src_wave = nullptr;

@@ -6,6 +6,8 @@ below on each axis, so an H source may reach it from one cell in front of a
 far slab; the step then has to keep the two routines apart.  The routines
 called one by one are the yardstick: the same operations in the same order,
 equal bit for bit."""
+import time
+
 import numpy as np
 import pytest
 
@@ -47,3 +49,34 @@ def test_sources_beside_a_slab_equal_the_routines(prec, axis, m):
             _same(_state(a), _state(b))
             a.close()
             b.close()
+
+
+def test_plain_calls_do_not_walk_the_sources():
+    """One step at a time costs what steps in one call cost, however many
+    sources there are: 50 calls with 200 000 sources, where a walk over them
+    takes milliseconds a call and a step's launches under a tenth of one."""
+    import cpsfdtd_b200 as cps
+    n, d = 72, 5e-9
+    dk = decks.Deck(n, n, n, d, d, d)
+    dk.pml = decks.pml_params(4)
+    g = cps.Grid.from_deck(dk, cps.FP32)
+    k, j, i = np.meshgrid(*[np.arange(7, 66)] * 3, indexing="ij")
+    at = np.stack([i.ravel(), j.ravel(), k.ravel()], axis=1)[:200000]
+    wave = np.ones(1)
+    for p in at.tolist():
+        g.source_add(decks.COMP["Ez"], *p, wave)
+
+    def ms(calls, steps):
+        best = 1e9
+        for _ in range(3):
+            g.sync()
+            t0 = time.perf_counter()
+            for _ in range(calls):
+                g.step(steps, cps.PLAIN)
+            g.sync()
+            best = min(best, 1e3 * (time.perf_counter() - t0))
+        return best
+
+    ms(1, 2)
+    one, many = ms(1, 50), ms(50, 1)
+    assert many < one + 25.0, (one, many)
