@@ -248,6 +248,17 @@ bool kernel_smem(int bytes, int carveout = -1)
     return smem_attr_once(done, reinterpret_cast<const void *>(K), bytes, carveout) == cudaSuccess;
 }
 
+// SMs of the device in use (the same on every device of a machine)
+inline int sm_count()
+{
+    static const int n = [] {
+        int dev = 0, v = 0;
+        cudaGetDevice(&dev);
+        return cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && v > 0 ? v : 1;
+    }();
+    return n;
+}
+
 // ------------------------------------------------------------ launchers
 // Plain path: one kernel per reference routine (kernels_plain.cu, built
 // without FMA contraction so FP64 results follow the reference roundings).

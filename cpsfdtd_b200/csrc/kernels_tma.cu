@@ -320,19 +320,23 @@ int h_tma_by(const GridMaps &M, const FieldView<T> &f, const PmlView<T> &p, int 
     }
 }
 
-}  // namespace
-
 // Planes per tile: as set, or the sweep's default, halved (to two at least)
-// while the grid has fewer tiles than the device holds at once (14 one-warp
-// tiles per SM, five block tiles).  A tile marches its planes one after the
-// other, so on a small grid the sweep takes the time of one tile: at 48^3, H
-// and E sweeps of 22 and 14 us with 16 and 8 planes.
-static int planes(int kc, const FusedShape &sh, const Dims &d, bool warp)
+// while the grid has fewer tiles than 14 per SM (one-warp tiles) or five (block
+// tiles of either height).  A tile marches its planes one after the other, so on
+// a small grid the sweep takes the time of one tile: at 48^3, H and E sweeps of
+// 22 and 14 us with 16 and 8 planes.  The line is measured.  It lies at about
+// one wave in FP32 (13 one-warp tiles fit an SM) and at two in FP64 (7 fit); with
+// the resident numbers in its place, us a step with CPML: 128^3 FP32 38.9 and
+// 45.2, 96^3 FP64 42.0 and 41.4, 112^3 FP64 69.6 and 73.5, 128^3 FP64 89.1 and
+// 86.3, other sizes from 36^3 to 176^3 within 1 %.
+int planes(int kc, const FusedShape &sh, const Dims &d, bool warp)
 {
-    const int64_t cols = (int64_t)cdiv(d.nx, 32) * cdiv(d.ny, sh.by), want = 148 * (warp ? 14 : 5);
+    const int64_t cols = (int64_t)cdiv(d.nx, 32) * cdiv(d.ny, sh.by), want = (int64_t)sm_count() * (warp ? 14 : 5);
     while (!sh.fixed && kc > 2 && cols * cdiv(d.nz, kc) < want) kc /= 2;
     return kc;
 }
+
+}  // namespace
 
 template <typename T>
 int launch_h_tma(const GridMaps &M, const FieldView<T> &f, const PmlView<T> &p, FusedShape sh, int *err,
