@@ -1066,7 +1066,6 @@ extern "C" cps_status cps_pml_init(cps_grid *g, const cps_pml_params *pp)
     }
     if ((s = dalloc(g, &g->d_pcoef, coef.size() * g->esz))) return s;
     if ((s = upload_real(g, g->d_pcoef, coef.data(), coef.size()))) return s;
-    const Dims &d = g->d;
     for (int f = 0; f < 6; ++f) {
         // each side's two words lie one after the other (one tensor map covers them)
         for (int q = 0; q < 4; q += 2)
@@ -1739,12 +1738,6 @@ extern "C" cps_status cps_step(cps_grid *g, int32_t nsteps, int32_t path)
 namespace cps {
 namespace {
 
-bool absorbed_kind(int k)
-{
-    return k == kOpHPml || k == kOpEPml || k == kOpDl || (k >= kOpGainP && k <= kOpGainN) ||
-           (k >= kOpThreeP && k <= kOpThreeN);
-}
-
 // Whether `ops` is a prefix (full = false) or a whole step (full = true) that
 // the fused sweeps reproduce.
 bool fusable(const cps_grid *g, const std::vector<RecOp> &ops, bool full)
@@ -2084,15 +2077,9 @@ extern "C" cps_status cps_grid_reset(cps_grid *g, int64_t n0)
     FLUSH_RECORDED(g);
     for (int c = 0; c < 6; ++c) CK(cudaMemsetAsync(g->F[c], 0, (size_t)g->elems * g->esz, g->stream));
     if (g->pml_on) {
-        const Dims &d = g->d;
-        for (int f = 0; f < 6; ++f) {
-            const int np = g->pml.npml[f];
-            size_t n;
-            if (f < 2) n = (size_t)(d.nz + 1) * (d.ny + 1) * psi_xw(np);
-            else if (f < 4) n = (size_t)(d.nz + 1) * (np + 1) * d.px;
-            else n = (size_t)(np + 1) * (d.ny + 1) * d.px;
-            for (int q = 0; q < 4; ++q) CK(cudaMemsetAsync(g->d_q[f][q], 0, n * g->esz, g->stream));
-        }
+        for (int f = 0; f < 6; ++f)
+            for (int q = 0; q < 4; ++q)
+                CK(cudaMemsetAsync(g->d_q[f][q], 0, psi_words(g, f) * g->esz, g->stream));
     }
     if (g->dl_on) CK(cudaMemsetAsync(g->d_dl_state, 0, (size_t)g->dl_n * 3 * g->dlc.stride * g->esz, g->stream));
     if (g->gain_on) {

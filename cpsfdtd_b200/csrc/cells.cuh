@@ -8,9 +8,6 @@
 
 namespace cps {
 
-template <typename T>
-__device__ __forceinline__ T ld(const T *p) { return __ldg(p); }
-
 // Coefficient of a cell's psi term.  By default the cell's own curl
 // coefficient: bE of its medium, the Drude-Lorentz C3 on ID-2 cells (p.ce_disp),
 // bH of its medium on the H side -- the CFS-PML update for any medium, and

@@ -12,19 +12,18 @@ namespace cps {
 
 namespace {
 
-// One block per tile of the launch's boxes.  PM selects the body: 0 the
-// CPML-free body for every tile, 1 the CPML body for every tile, 2 the body
-// each tile needs (tile_in_pml).  Sweeps without gain run one launch (PM 2).
-// An FP32 sweep with gain (its gain words staged with the fields) runs every
-// tile on the CPML body in one launch (PM 1; the body leaves cells outside
-// the slabs as the CPML-free body would, bit for bit): measured faster than
-// CPML and interior tiles as two launches at every grid size tried, 128^3 to
-// 384^3, since a second launch's partial last wave costs more than the
-// interior blocks gain from the CPML-free body's lower register count.  An
-// FP64 sweep with gain (gain words read on the cell list) keeps the two
-// launches, so its interior blocks are not held to the CPML body's registers.
-template <typename T, int BY, int PM, bool DL, bool GAIN>
-__global__ void __launch_bounds__(32 * BY, GAIN ? 512 / (32 * BY) : 1024 / (32 * BY))
+// E sweep with gain (block tiles): one block per tile of the launch's boxes,
+// every tile on the CPML body (PML) or on the CPML-free one.  In FP32 (gain
+// words staged with the fields) one launch runs every tile of a grid with CPML
+// on the CPML body (it leaves cells outside the slabs as the CPML-free body
+// would, bit for bit): measured faster than CPML and interior tiles as two
+// launches at every grid size tried, 128^3 to 384^3, since a second launch's
+// partial last wave costs more than the interior blocks gain from the CPML-free
+// body's lower register count.  In FP64 (gain words read on the cell list) the
+// two launches stay, so its interior blocks are not held to the CPML body's
+// registers.
+template <typename T, int BY, bool PML, bool DL>
+__global__ void __launch_bounds__(32 * BY, 512 / (32 * BY))
     k_e_tma(const __grid_constant__ TmaMaps M, FieldView<T> f, PmlView<T> p, DlView<T> D, GainView<T> G, int kc,
             const __grid_constant__ TileBoxes tb, int *err)
 {
@@ -41,14 +40,12 @@ __global__ void __launch_bounds__(32 * BY, GAIN ? 512 / (32 * BY) : 1024 / (32 *
     init_stages(full);
     pdl_wait();
     uint32_t ctr = 0;
-    if (PM == 1 || (PM == 2 && tile_in_pml(p.np, f.d, t.bx * 32, t.by * BY, BY, k0, k1, true)))
-        e_tma_body<T, BY, PM != 0, DL, GAIN>(M, f, p, D, G, kc, t, ctr, err, sm, full);
-    else
-        e_tma_body<T, BY, false, DL, GAIN>(M, f, p, D, G, kc, t, ctr, err, sm, full);
+    e_tma_body<T, BY, PML, DL, true>(M, f, p, D, G, kc, t, ctr, err, sm, full);
 }
 
-// FP64 H sweep (block tiles): one launch, the body each tile needs (PM 2)
-template <typename T, int BY, int PM>
+// FP64 H sweep (block tiles): one launch; on a grid with CPML (PML) the body each
+// tile needs
+template <typename T, int BY, bool PML>
 __global__ void __launch_bounds__(32 * BY) k_h_tma(const __grid_constant__ TmaMaps M, FieldView<T> f, PmlView<T> p,
                                                     int kc, const __grid_constant__ TileBoxes tb, int *err)
 {
@@ -65,8 +62,8 @@ __global__ void __launch_bounds__(32 * BY) k_h_tma(const __grid_constant__ TmaMa
     init_stages(full);
     pdl_wait();
     uint32_t ctr = 0;
-    if (PM == 1 || (PM == 2 && tile_in_pml(p.np, f.d, t.bx * 32, t.by * BY, BY, k0, k1, false)))
-        h_tma_body<T, BY, PM != 0>(M, f, p, kc, t, ctr, err, sm, full);
+    if (PML && tile_in_pml(p.np, f.d, t.bx * 32, t.by * BY, BY, k0, k1, false))
+        h_tma_body<T, BY, PML>(M, f, p, kc, t, ctr, err, sm, full);
     else
         h_tma_body<T, BY, false>(M, f, p, kc, t, ctr, err, sm, full);
 }
@@ -78,8 +75,8 @@ constexpr int warp_blocks()
     return (227 * 1024) / (warp_ring<T, BY>() + 1024 + 640);
 }
 
-// One warp per tile.  PM: 0 no CPML on the grid, 2 the body each tile needs.
-template <typename T, int BY, int PM>
+// One warp per tile; on a grid with CPML (PML) the body each tile needs.
+template <typename T, int BY, bool PML>
 __global__ void __launch_bounds__(32, warp_blocks<T, BY>())
     k_h_warp(const __grid_constant__ SweepMaps M, FieldView<T> f, PmlView<T> p, int kc, int nbx, int nby, int *err)
 {
@@ -97,13 +94,13 @@ __global__ void __launch_bounds__(32, warp_blocks<T, BY>())
     init_ring(full);
     pdl_wait();
     Ring R{align_smem(sm_raw), full, warp_ring<T, BY>() - 128, 0u, wait_skew(err), err};
-    if (PM == 1 || (PM == 2 && tile_in_pml(p.np, f.d, t.bx * 32, t.by * BY, BY, k0, k1, false)))
-        h_warp_tile<T, BY, 1, PM != 0>(M, f, p, kc, t, R, tab);
+    if (PML && tile_in_pml(p.np, f.d, t.bx * 32, t.by * BY, BY, k0, k1, false))
+        h_warp_tile<T, BY, 1, PML>(M, f, p, kc, t, R, tab);
     else
         h_warp_tile<T, BY, kPlanes, false>(M, f, p, kc, t, R, tab);
 }
 
-template <typename T, int BY, int PM, bool DL>
+template <typename T, int BY, bool PML, bool DL>
 __global__ void __launch_bounds__(32, warp_blocks<T, BY>())
     k_e_warp(const __grid_constant__ SweepMaps M, FieldView<T> f, PmlView<T> p, int kc, int nbx, int nby, int *err)
 {
@@ -121,8 +118,8 @@ __global__ void __launch_bounds__(32, warp_blocks<T, BY>())
     init_ring(full);
     pdl_wait();
     Ring R{align_smem(sm_raw), full, warp_ring<T, BY>() - 128, 0u, wait_skew(err), err};
-    if (PM == 1 || (PM == 2 && tile_in_pml(p.np, f.d, t.bx * 32, t.by * BY, BY, k0, k1, true)))
-        e_warp_tile<T, BY, 1, PM != 0, DL>(M, f, p, kc, t, R, tab);
+    if (PML && tile_in_pml(p.np, f.d, t.bx * 32, t.by * BY, BY, k0, k1, true))
+        e_warp_tile<T, BY, 1, PML, DL>(M, f, p, kc, t, R, tab);
     else
         e_warp_tile<T, BY, kPlanes, false, DL>(M, f, p, kc, t, R, tab);
 }
@@ -216,49 +213,49 @@ inline SweepTiles sweep_tiles(const int np[6], bool pml_on, const Dims &d, int b
     return t;
 }
 
-template <typename T, int BY, int PM, bool DL, bool GAIN>
+template <typename T, int BY, bool PML, bool DL>
 int e_tma_launch(const TmaMaps &M, const FieldView<T> &f, const PmlView<T> &p, const DlView<T> &D,
                  const GainView<T> &G, int kc, const TileBoxes &tb, int *err, cudaStream_t s)
 {
-    using L = ELayout<T, BY, GAIN>;
+    using L = ELayout<T, BY, true>;
     const int blocks = tb.start[tb.n];
     if (blocks <= 0) return 0;
-    if (!set_smem<k_e_tma<T, BY, PM, DL, GAIN>>(L::SMEM)) return 0;
-    launch_pdl(!DL, k_e_tma<T, BY, PM, DL, GAIN>, blocks, dim3(32, BY), L::SMEM, s, M, f, p, D, G, kc, tb, err);
+    if (!set_smem<k_e_tma<T, BY, PML, DL>>(L::SMEM)) return 0;
+    launch_pdl(!DL, k_e_tma<T, BY, PML, DL>, blocks, dim3(32, BY), L::SMEM, s, M, f, p, D, G, kc, tb, err);
     return 1;
 }
 
-template <typename T, int BY, int PM>
+template <typename T, int BY, bool PML>
 int h_tma_launch(const TmaMaps &M, const FieldView<T> &f, const PmlView<T> &p, int kc, const TileBoxes &tb,
                  int *err, cudaStream_t s)
 {
     using L = StageLayout<T, BY>;
     const int blocks = tb.start[tb.n];
     if (blocks <= 0) return 0;
-    if (!set_smem<k_h_tma<T, BY, PM>>(L::SMEM)) return 0;
-    launch_pdl(true, k_h_tma<T, BY, PM>, blocks, dim3(32, BY), L::SMEM, s, M, f, p, kc, tb, err);
+    if (!set_smem<k_h_tma<T, BY, PML>>(L::SMEM)) return 0;
+    launch_pdl(true, k_h_tma<T, BY, PML>, blocks, dim3(32, BY), L::SMEM, s, M, f, p, kc, tb, err);
     return 1;
 }
 
-template <typename T, int BY, int PM>
+template <typename T, int BY, bool PML>
 int h_warp_launch(const SweepMaps &M, const FieldView<T> &f, const PmlView<T> &p, int kc, int *err, cudaStream_t s)
 {
     kc = (kc + kPlanes - 1) / kPlanes * kPlanes;
     constexpr int smem = warp_ring<T, BY>();
     const int nbx = (int)cdiv(f.d.nx, 32), nby = (int)cdiv(f.d.ny, BY), nbz = (int)cdiv(f.d.nz, kc);
-    if (!set_smem<k_h_warp<T, BY, PM>>(smem)) return 0;
-    launch_pdl(true, k_h_warp<T, BY, PM>, nbx * nby * nbz, 32, smem, s, M, f, p, kc, nbx, nby, err);
+    if (!set_smem<k_h_warp<T, BY, PML>>(smem)) return 0;
+    launch_pdl(true, k_h_warp<T, BY, PML>, nbx * nby * nbz, 32, smem, s, M, f, p, kc, nbx, nby, err);
     return 1;
 }
 
-template <typename T, int BY, int PM, bool DL>
+template <typename T, int BY, bool PML, bool DL>
 int e_warp_launch(const SweepMaps &M, const FieldView<T> &f, const PmlView<T> &p, int kc, int *err, cudaStream_t s)
 {
     kc = (kc + kPlanes - 1) / kPlanes * kPlanes;
     constexpr int smem = warp_ring<T, BY>();
     const int nbx = (int)cdiv(f.d.nx, 32), nby = (int)cdiv(f.d.ny, BY), nbz = (int)cdiv(f.d.nz, kc);
-    if (!set_smem<k_e_warp<T, BY, PM, DL>>(smem)) return 0;
-    launch_pdl(!DL, k_e_warp<T, BY, PM, DL>, nbx * nby * nbz, 32, smem, s, M, f, p, kc, nbx, nby, err);
+    if (!set_smem<k_e_warp<T, BY, PML, DL>>(smem)) return 0;
+    launch_pdl(!DL, k_e_warp<T, BY, PML, DL>, nbx * nby * nbz, 32, smem, s, M, f, p, kc, nbx, nby, err);
     return 1;
 }
 
@@ -269,20 +266,20 @@ void attrs_by()
     constexpr int S = warp_ring<T, BY>(), SB = StageLayout<T, BY>::SMEM;
     constexpr int SG = ELayout<T, BY, true>::SMEM;
     if constexpr (sizeof(T) == 4) {
-        set_smem<k_h_warp<T, BY, 0>>(S);
-        set_smem<k_h_warp<T, BY, 2>>(S);
+        set_smem<k_h_warp<T, BY, false>>(S);
+        set_smem<k_h_warp<T, BY, true>>(S);
     } else {
-        set_smem<k_h_tma<T, BY, 0>>(SB);
-        set_smem<k_h_tma<T, BY, 2>>(SB);
+        set_smem<k_h_tma<T, BY, false>>(SB);
+        set_smem<k_h_tma<T, BY, true>>(SB);
     }
-    set_smem<k_e_warp<T, BY, 0, false>>(S);
-    set_smem<k_e_warp<T, BY, 0, true>>(S);
-    set_smem<k_e_warp<T, BY, 2, false>>(S);
-    set_smem<k_e_warp<T, BY, 2, true>>(S);
-    set_smem<k_e_tma<T, BY, 0, false, true>>(SG);
-    set_smem<k_e_tma<T, BY, 0, true, true>>(SG);
-    set_smem<k_e_tma<T, BY, 1, false, true>>(SG);
-    set_smem<k_e_tma<T, BY, 1, true, true>>(SG);
+    set_smem<k_e_warp<T, BY, false, false>>(S);
+    set_smem<k_e_warp<T, BY, false, true>>(S);
+    set_smem<k_e_warp<T, BY, true, false>>(S);
+    set_smem<k_e_warp<T, BY, true, true>>(S);
+    set_smem<k_e_tma<T, BY, false, false>>(SG);
+    set_smem<k_e_tma<T, BY, false, true>>(SG);
+    set_smem<k_e_tma<T, BY, true, false>>(SG);
+    set_smem<k_e_tma<T, BY, true, true>>(SG);
 }
 
 template <typename T, int BY>
@@ -292,21 +289,21 @@ int e_tma_by(const GridMaps &M, const FieldView<T> &f, const PmlView<T> &p, cons
     const bool dl = D.on && D.ncell > 0, gn = G.on && G.ncell > 0;
     if (gn && sizeof(T) == 4 && p.on) {  // every tile on the CPML body, one launch
         const TileBoxes all = whole_grid(f.d, BY, kc);
-        return dl ? e_tma_launch<T, BY, 1, true, true>(M.t, f, p, D, G, kc, all, err, s)
-                  : e_tma_launch<T, BY, 1, false, true>(M.t, f, p, D, G, kc, all, err, s);
+        return dl ? e_tma_launch<T, BY, true, true>(M.t, f, p, D, G, kc, all, err, s)
+                  : e_tma_launch<T, BY, true, false>(M.t, f, p, D, G, kc, all, err, s);
     }
     if (gn) {  // CPML tiles (if any) and interior tiles as two launches
         const SweepTiles t = sweep_tiles(p.np, p.on, f.d, BY, kc, true);
-        return (dl ? e_tma_launch<T, BY, 1, true, true>(M.t, f, p, D, G, kc, t.pml, err, s)
-                   : e_tma_launch<T, BY, 1, false, true>(M.t, f, p, D, G, kc, t.pml, err, s)) +
-               (dl ? e_tma_launch<T, BY, 0, true, true>(M.t, f, p, D, G, kc, t.interior, err, s)
-                   : e_tma_launch<T, BY, 0, false, true>(M.t, f, p, D, G, kc, t.interior, err, s));
+        return (dl ? e_tma_launch<T, BY, true, true>(M.t, f, p, D, G, kc, t.pml, err, s)
+                   : e_tma_launch<T, BY, true, false>(M.t, f, p, D, G, kc, t.pml, err, s)) +
+               (dl ? e_tma_launch<T, BY, false, true>(M.t, f, p, D, G, kc, t.interior, err, s)
+                   : e_tma_launch<T, BY, false, false>(M.t, f, p, D, G, kc, t.interior, err, s));
     }
     if (p.on)
-        return dl ? e_warp_launch<T, BY, 2, true>(M.e, f, p, kc, err, s)
-                  : e_warp_launch<T, BY, 2, false>(M.e, f, p, kc, err, s);
-    return dl ? e_warp_launch<T, BY, 0, true>(M.e, f, p, kc, err, s)
-              : e_warp_launch<T, BY, 0, false>(M.e, f, p, kc, err, s);
+        return dl ? e_warp_launch<T, BY, true, true>(M.e, f, p, kc, err, s)
+                  : e_warp_launch<T, BY, true, false>(M.e, f, p, kc, err, s);
+    return dl ? e_warp_launch<T, BY, false, true>(M.e, f, p, kc, err, s)
+              : e_warp_launch<T, BY, false, false>(M.e, f, p, kc, err, s);
 }
 
 template <typename T, int BY>
@@ -314,9 +311,9 @@ int h_tma_by(const GridMaps &M, const FieldView<T> &f, const PmlView<T> &p, int 
 {
     if constexpr (sizeof(T) == 8) {
         const TileBoxes all = whole_grid(f.d, BY, kc);
-        return p.on ? h_tma_launch<T, BY, 2>(M.t, f, p, kc, all, err, s) : h_tma_launch<T, BY, 0>(M.t, f, p, kc, all, err, s);
+        return p.on ? h_tma_launch<T, BY, true>(M.t, f, p, kc, all, err, s) : h_tma_launch<T, BY, false>(M.t, f, p, kc, all, err, s);
     } else {
-        return p.on ? h_warp_launch<T, BY, 2>(M.h, f, p, kc, err, s) : h_warp_launch<T, BY, 0>(M.h, f, p, kc, err, s);
+        return p.on ? h_warp_launch<T, BY, true>(M.h, f, p, kc, err, s) : h_warp_launch<T, BY, false>(M.h, f, p, kc, err, s);
     }
 }
 

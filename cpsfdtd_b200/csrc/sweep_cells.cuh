@@ -86,44 +86,6 @@ __device__ __forceinline__ ColPml<T> col_pml_h(const PmlView<T> &p, const Dims &
     return c;
 }
 
-// CPML H corrections at one cell (CPML.cpp:617-682), x then y then z slabs
-template <typename T>
-__device__ __forceinline__ void pml_h_cell(const PmlView<T> &p, const Dims &d, const ColPml<T> &c, T ch, int i,
-                                           int j, int k, T dEz_i, T dEy_i, T dEx_j, T dEz_j, T dEy_k, T dEx_k, T &hx,
-                                           T &hy, T &hz)
-{
-    if (c.fx >= 0) {
-        const int np = p.np[c.fx];
-        const int64_t q = ((int64_t)k * (d.ny + 1) + j) * psi_xw(np) + c.sxl;
-        T *q0 = p.qh[c.fx][0], *q1 = p.qh[c.fx][1];
-        const T a0 = c.bx * q0[q] + c.cx * dEz_i, a1 = c.bx * q1[q] + c.cx * dEy_i;
-        q0[q] = a0; q1[q] = a1;
-        hy = hy + a0 * ch;
-        hz = hz - a1 * ch;
-    }
-    if (c.fy >= 0) {
-        const int np = p.np[c.fy];
-        const int64_t q = ((int64_t)k * (np + 1) + c.syl) * d.px + i;
-        T *q0 = p.qh[c.fy][0], *q1 = p.qh[c.fy][1];
-        const T a0 = c.by * q0[q] + c.cy * dEx_j, a1 = c.by * q1[q] + c.cy * dEz_j;
-        q0[q] = a0; q1[q] = a1;
-        hz = hz - a0 * ch;
-        hx = hx + a1 * ch;
-    }
-    int fz = -1, szl = 0;
-    if (k < p.np[kFZ1]) { fz = kFZ1; szl = k; }
-    else if (k >= d.nz - p.np[kFZ2]) { fz = kFZ2; szl = k - (d.nz - p.np[kFZ2]); }
-    if (fz >= 0) {
-        const int64_t q = ((int64_t)szl * (d.ny + 1) + j) * d.px + i;
-        T *q0 = p.qh[fz][0], *q1 = p.qh[fz][1];
-        const T b = p.bH[fz][szl], cc = p.cH[fz][szl];
-        const T a0 = b * q0[q] + cc * dEy_k, a1 = b * q1[q] + cc * dEx_k;
-        q0[q] = a0; q1[q] = a1;
-        hx = hx - a0 * ch;
-        hy = hy + a1 * ch;
-    }
-}
-
 // CPML E corrections at one cell (CPML.cpp:537-602), x then y then z slabs
 template <typename T>
 __device__ __forceinline__ void pml_e_cell(const PmlView<T> &p, const Dims &d, const ColPml<T> &c, T ce, int i,
@@ -192,7 +154,7 @@ __device__ __forceinline__ void psi_load_e(const PmlView<T> &p, const Dims &d, c
     }
 }
 
-// H-side psi of plane k for a column (slab membership as in pml_h_cell)
+// H-side psi of plane k for a column (slabs [0, np-1] and [n-np, n-1])
 template <typename T>
 __device__ __forceinline__ void psi_load_h(const PmlView<T> &p, const Dims &d, const ColPml<T> &c, int i, int j, int k,
                                            PsiRegs<T> &r)
@@ -247,8 +209,8 @@ __device__ __forceinline__ void pml_e_cell_pre(const PmlView<T> &p, const Dims &
     }
 }
 
-// CPML H corrections with psi already in registers (same arithmetic as
-// pml_h_cell); STORE = false computes the corrected H without writing psi
+// CPML H corrections (CPML.cpp:617-682), x then y then z slabs, with psi already
+// in registers; STORE = false computes the corrected H without writing psi
 template <typename T, bool STORE = true>
 __device__ __forceinline__ void pml_h_cell_pre(const PmlView<T> &p, const Dims &d, const ColPml<T> &c, T ch, int i,
                                                int j, int k, const PsiRegs<T> &r, T dEz_i, T dEy_i, T dEx_j, T dEz_j,
@@ -305,30 +267,6 @@ __device__ __forceinline__ T dl_component_regs(const DlCoef<T> &D, T E, T curl, 
     }
     st[(ND + 2 * NL) * sc] = temp;
     return E;
-}
-
-// Drude-Lorentz update of the ID-2 cells of a warp row (ballot-ranked lookup
-// into the compacted list); the whole warp must call it
-template <typename T>
-__device__ __forceinline__ void dl_warp(const DlView<T> &D, const Dims &d, int j, int k, int seg, bool act, int id,
-                                        T dHz_j, T dHy_k, T dHx_k, T dHz_i, T dHy_i, T dHx_j, T cExy, T cEyx,
-                                        T cExz, T cEyz, T cEzy, T cEzx, T &ex, T &ey, T &ez)
-{
-    const bool mine = act && id == CPS_ID_DISPERSIVE;
-    const unsigned m = __ballot_sync(0xffffffffu, mine);
-    if (!m) return;
-    const int nseg = d.px >> 5;
-    const int64_t base = D.seg[((int64_t)k * (d.ny + 1) + j) * nseg + seg];
-    if (!mine) return;
-    const int64_t c = base + __popc(m & lanemask_lt()), sc = D.ncell;
-    const T C3 = D.c.C3;
-    const T cxx = C3 * dHz_j * cExz - C3 * dHy_k * cExy;
-    const T cyy = C3 * dHx_k * cEyx - C3 * dHz_i * cEyz;
-    const T czz = C3 * dHy_i * cEzy - C3 * dHx_j * cEzx;
-    T *st = D.state + c;
-    ex = dl_component(D.c, ex, cxx, st, sc);
-    ey = dl_component(D.c, ey, cyy, st + (int64_t)D.c.stride * sc, sc);
-    ez = dl_component(D.c, ez, czz, st + (int64_t)2 * D.c.stride * sc, sc);
 }
 
 // four-level gain P -> E -> N at the gain cells of a warp row; the whole warp
