@@ -4,14 +4,16 @@
 // is built with the one-grid C ABI and keeps its own state, step counter and
 // results, which the one-grid calls read as usual.
 //
-// A step of the batch is one launch per sweep class (H interior / H CPML
-// tiles; E interior / E CPML tiles, each with and without gain) over flat
-// tables of tiles that name their grid, then the Drude-Lorentz cells, TF/SF
-// injection, sources and port sampling of all grids, each one launch.  Steps
-// run in chunks of at most kMaxRing; a chunk ends with one port-DFT
+// A step of the batch sweeps every member with the one-grid kernels, spread over
+// side streams (the default, and always for members of kBigCells or more), or
+// all members' tiles in one launch per sweep class (H interior / H CPML tiles;
+// E interior / E CPML tiles, each with and without gain) over flat tables of
+// tiles that name their grid.  TF/SF injection, sources and port sampling of all
+// grids are one launch each; a batch of one grid takes its pointers as kernel
+// parameters there, not through tables.  Steps run in chunks of at most kMaxRing; a chunk ends with one port-DFT
 // contraction over every port and a kernel that advances every grid's step
-// counter, and is captured once into a CUDA graph per chunk length and
-// replayed while the membership and tiling stay the same.
+// counter, and is captured into a CUDA graph per chunk length when that length
+// comes a second time, and replayed while the membership and tiling stay the same.
 #include <math.h>
 #include <stdio.h>
 #include <string.h>

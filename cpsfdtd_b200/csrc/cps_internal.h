@@ -341,8 +341,8 @@ void launch_e_fused(const FieldView<T> &f, const PmlView<T> &p, const DlView<T> 
 }  // namespace cps
 #include "tma.cuh"
 namespace cps {
-// (each sweep launches its CPML tiles and its interior tiles separately;
-// the return value is the number of kernels launched)
+// (one launch per sweep, an FP64 E sweep with gain two: its CPML tiles and its
+// interior tiles; the return value is the number of kernels launched)
 template <typename T>
 int launch_h_tma(const GridMaps &M, const FieldView<T> &f, const PmlView<T> &p, FusedShape sh, int *err,
                  cudaStream_t s);

@@ -76,14 +76,15 @@ __global__ void k_phasors(const double *omega, int nfreq, int nslots, int64_t n_
 // fused multiply-adds) in slot order, so every accumulator sees the same
 // operations in the same order whatever the tile.
 //
-// Bound: the FP64 pipe, then the accumulators' round trip to DRAM.  Eight
-// points per phasor read keep shared memory below the pipe (a 16-byte read
-// serves 16 multiply-adds; 4 x 4 tiles would need 20 cycles of reads for 16),
-// the frequency tile follows the port (a tile of 32 does four times the work
-// for eight frequencies), and three blocks per SM let one load or store its
-// accumulators while others contract.  64 slots, FP32 samples, all ports of the
-// grid: 256^3 with 16 frequencies 892 -> 346 us, 384^3 with 8 2159 -> 595 us,
-// sixteen grids with 16 1500 -> 577 us.
+// Bound: latency at twelve warps per SM (three blocks, 168 registers): 256^3 with
+// 64 frequencies keeps the FP64 pipe 40 % busy, shared memory 26 %, the
+// conversions' pipe 20 %.  Eight points per phasor read keep shared memory below
+// the pipe (a 16-byte read serves 16 multiply-adds; 4 x 4 tiles would need 20
+// cycles of reads for 16), the frequency tile follows the port (a tile of 32 does
+// four times the work for eight frequencies), and three blocks per SM let one load
+// or store its accumulators while others contract.  64 slots, FP32 samples, all
+// ports of the grid: 256^3 with 16 frequencies 892 -> 346 us, 384^3 with 8 2159 ->
+// 595 us, sixteen grids with 16 1500 -> 577 us.
 constexpr int kMaxSlots = 64, kDftThreads = 128, kDftPoints = 8;
 constexpr int kDftStage = 16384;  // bytes of a sample buffer
 constexpr size_t kDftSmem = 2 * kDftStage + sizeof(double2) * 16 * kMaxSlots;

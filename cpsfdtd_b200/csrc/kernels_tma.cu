@@ -1,5 +1,7 @@
 // kernels_tma.cu -- one-grid launches of the TMA-fed fused H and E sweeps
-// (sm_100a): one block per 32 x BY x kc tile, bodies in tma_bodies.cuh.
+// (sm_100a), one 32 x BY x kc tile per block: one-warp tiles (warp_tiles.cuh) for
+// FP32 H sweeps and E sweeps without gain, block tiles (tma_bodies.cuh) for FP64
+// H sweeps and E sweeps with gain.
 #include <cuda.h>
 #include <string.h>
 

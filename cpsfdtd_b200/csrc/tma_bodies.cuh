@@ -3,7 +3,7 @@
 // over many grids (kernels_batch.cu).
 //
 // A tile is a 32 x BY block of (i, j) columns marching planes [k0, k1) in k.
-// Thread 0 keeps kStages planes of x-y tiles in flight: for each plane one
+// Thread 0 keeps up to kStages planes of x-y tiles in flight: for each plane one
 // mbarrier, and cp.async.bulk.tensor loads of
 //   E sweep: H with a one-cell low halo (box 36 x (BY+1) from (x0-4, y0-1)),
 //            E and the uint8 ID of the tile (box 32 x BY from (x0, y0));
@@ -12,9 +12,9 @@
 // The x origin of every box is a multiple of 4 elements (16 bytes); boxes
 // that reach outside the arrays read zeros.  No multicast is used.
 // Threads take their cell and its x/y neighbours from the staged tile and the
-// k-neighbour from registers, update, and store with plain coalesced stores;
-// when all threads are done with a stage (__syncthreads) thread 0 refills it
-// with the plane kStages ahead.
+// k-neighbour from registers, update, and store with plain coalesced stores.
+// One block barrier per plane: past the one at plane k all threads are done with
+// plane k - 1, whose stage thread 0 then refills with plane k - 1 + kStages.
 //
 // Stage bookkeeping runs on a block-uniform counter `ctr` of planes that went
 // through the ring, so a block may run several tiles in a row (persistent
@@ -153,9 +153,10 @@ __device__ __forceinline__ bool tile_in_pml(const int np[6], const Dims &d, int 
 }
 
 // Up to six boxes of tiles (in tile coordinates) covered by one launch, one
-// block per tile: a sweep launches its interior tiles (one box, the CPML-free
-// body) and its CPML tiles (the rest of the grid, up to six boxes) separately,
-// so the interior blocks are not held to the CPML body's register count.
+// block per tile: the whole grid as one box, or, in the FP64 E sweep with gain,
+// the interior tiles (one box, the CPML-free body) and the CPML tiles (the rest
+// of the grid, up to six boxes) as two launches, so that the interior blocks are
+// not held to the CPML body's register count.
 struct TileBoxes {
     int n;         // boxes in use
     int start[7];  // first block of each box; start[n] = blocks in the launch

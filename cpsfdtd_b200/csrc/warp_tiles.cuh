@@ -19,8 +19,8 @@
 // lane, and broadcast by shuffles.
 //
 // Measured against block tiles with one cell per thread (B200, FP32, CPML):
-// 301x419x262, H sweep 262 -> 235 us and E sweep 287 -> 228 us (DRAM at 73 % of
-// its peak, 5.96 TB/s); 256^3 dispersive, H 147 -> 127 us; 384^3 laser, H 424 ->
+// 301x419x262, H sweep 262 -> 235 us and E sweep 287 -> 228 us (DRAM at 76 % of
+// its peak, 1.41 GB a sweep); 256^3 dispersive, H 147 -> 127 us; 384^3 laser, H 424 ->
 // 380 us.  E sweeps with gain stay on block tiles (a lane with four cells' gain
 // words leaves six warps per SM: 1407 us either way at 384^3, 6 % slower at
 // 150x117x98), and so does the FP64 H sweep (90 against 100 us at 165x150x181).

@@ -283,12 +283,18 @@ CPS_API cps_status cps_grid_set_step(cps_grid *g, int64_t n);
 CPS_API cps_status cps_grid_get_step(const cps_grid *g, int64_t *n);
 /* advance nsteps steps, each in the order of main.cpp:267-344: H bulk, TF/SF H,
  * CPML H, E bulk, Drude-Lorentz, gain (P, E, N), TF/SF E, sources, CPML E,
- * port sampling.  Asynchronous on the grid's stream. */
+ * port sampling.  Asynchronous on the grid's stream (a call that makes the
+ * tables of the grid's chunks, below, waits for it once).  On the fused path
+ * sources are added after the E sweep and its CPML terms, which so see an H
+ * source in a slab, or one cell in front of a far one, a step later. */
 CPS_API cps_status cps_step(cps_grid *g, int32_t nsteps, int32_t path);
-/* On (default): cps_step on the fused path runs grids of 4 Mi cells or more
- * as chunks of a one-grid batch (the batch's CUDA-graph-replayed chunks; the
- * results are the direct launches' bit for bit), except while per-step timing
- * (cps_grid_set_timing) is on; off: one launch sequence per step. */
+/* On (default): cps_step on the fused path runs in chunks of a one-grid batch
+ * (the batch's CUDA-graph-replayed chunks; the results are the direct launches'
+ * bit for bit): every call on a grid of 4 Mi cells or more, and on a smaller one
+ * the first call of 32 steps or more and from then on those long enough to pay
+ * for folding the grid's port DFTs at their end.  One launch sequence per step
+ * while per-step timing (cps_grid_set_timing) is on, while the caller captures
+ * the grid's stream, and with this off. */
 CPS_API cps_status cps_grid_set_chunked(cps_grid *g, int32_t on);
 
 /* ---- single reference routines (one launch each, enqueued on the grid's stream) ---- */
@@ -378,9 +384,10 @@ CPS_API cps_status cps_ports_flush(cps_grid *g);
  * milliseconds.  stride 0 turns it off and clears the samples. */
 CPS_API cps_status cps_grid_set_timing(cps_grid *g, int32_t stride);
 /* tile of the fused sweeps: rows (4, 8 or 16) of 32 columns per block and
- * planes marched per block (>= 1), set for every sweep; the default is 4 rows
- * with 8 planes for the E sweep, 16 for the H sweep and 4 for an FP32 E sweep
- * with gain.  cps_grid_get_tile returns the rows and the E sweep's planes.
+ * planes marched per tile (>= 1), set for every sweep; the default is 4 rows
+ * with 8 planes, 16 for an FP64 H sweep and 4 for an FP32 E sweep with gain,
+ * fewer on grids whose tiles would not fill the device.  In a cps_batch the
+ * batch's rows hold.  cps_grid_get_tile returns the rows and the E sweep's planes.
  * Tiling does not change results. */
 CPS_API cps_status cps_grid_set_tile(cps_grid *g, int32_t rows, int32_t planes);
 CPS_API cps_status cps_grid_get_tile(const cps_grid *g, int32_t *rows, int32_t *planes);
