@@ -508,7 +508,7 @@ cps_status run_chunk(cps_batch *b, int S)
         if (e != cudaSuccess) {
             cudaGetLastError();
             set_error(std::string("batch graph instantiation failed: ") + cudaGetErrorString(e));
-            return CPS_E_CUDA;
+            return e == cudaErrorMemoryAllocation ? CPS_E_NOMEM : CPS_E_CUDA;
         }
         it = b->graphs.insert({S, {exec, n}}).first;
     }
@@ -550,7 +550,10 @@ cps_status step_batch_T(cps_batch *b, int nsteps)
     while (nsteps > 0) {
         const int S = std::min(nsteps, kMaxRing);
         if (b->graph && S != kMaxRing && b->graphs.find(S) == b->graphs.end() && b->graphs.size() > 8) drop_graphs(b);
-        if ((s = run_chunk<T>(b, S))) return s;
+        if ((s = run_chunk<T>(b, S))) {
+            sync_grid_streams_out(b);  // the chunks before it
+            return s;
+        }
         for (cps_grid *g : b->grids) {
             g->step += S;
             for (PortState &P : g->ports) {
@@ -644,7 +647,7 @@ extern "C" cps_status cps_batch_create(int32_t precision, cps_batch **out)
         if (b->stream) cudaStreamDestroy(b->stream);
         delete b;
         set_error(std::string("cps_batch_create: ") + cudaGetErrorString(e));
-        return CPS_E_CUDA;
+        return e == cudaErrorMemoryAllocation ? CPS_E_NOMEM : CPS_E_CUDA;
     }
     *out = b;
     return CPS_OK;

@@ -1717,7 +1717,12 @@ extern "C" cps_status cps_step(cps_grid *g, int32_t nsteps, int32_t path)
     REQUIRE(path == CPS_PATH_PLAIN || path == CPS_PATH_FUSED || path == CPS_PATH_ONEPASS, CPS_E_INVALID,
             "cps_step: unknown path");
     CK(cudaSetDevice(g->desc.device));
-    if (path == CPS_PATH_FUSED && nsteps > 0 && solo_eligible(g, nsteps)) return solo_step(g, nsteps);
+    if (path == CPS_PATH_FUSED && nsteps > 0 && solo_eligible(g, nsteps)) {
+        const int64_t n0 = g->step;
+        s = solo_step(g, nsteps);
+        if (s != CPS_E_NOMEM) return s;
+        nsteps -= (int32_t)(g->step - n0);  // no room for the chunks' tables or graphs: one launch after another
+    }
     return g->fp32 ? step_T<float>(g, nsteps, path) : step_T<double>(g, nsteps, path);
 }
 
