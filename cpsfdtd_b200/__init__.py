@@ -404,7 +404,7 @@ class Grid:
         _check(self.L.cps_synchronize(self.h))
 
     def set_chunked(self, on):
-        """fused steps of large grids as graph-replayed one-grid batch chunks (default on)"""
+        """fused steps as graph-replayed one-grid batch chunks where that pays (default on)"""
         _check(self.L.cps_grid_set_chunked(self.h, 1 if on else 0))
 
     def reset(self, n0=1):
@@ -580,7 +580,8 @@ class Batch:
         """Tile rows (4 or 8), planes per tile and sweep launch mode: 0 one
         launch per sweep class, one block per tile; 1 the same, persistent;
         2 each member's own launches on side streams (the default, with
-        4 rows and 16 planes).  Results do not depend on the choice."""
+        4 rows, the members' own planes and 16 in FP32 E sweeps with gain until
+        this sets them).  Results do not depend on the choice."""
         _check(self.L.cps_batch_set_tile(self.h, rows, planes, persistent))
 
     def get_tile(self):
